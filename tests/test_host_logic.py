@@ -208,6 +208,55 @@ def test_vllm_v1_backend_conforms_to_the_installed_interface():
     assert builder.layer_names == ["l0"]
 
 
+class _StandInStore:
+    """Records the calls that the v1 backend makes of its store; nothing is computed."""
+
+    record_bytes, device = 2 * 64 * 6 + 128, torch.device("cpu")
+
+    def __init__(self):
+        self.calls = []
+
+    def append(self, pool, key, value, rowmap):
+        self.calls.append(("append", key.shape[0]))
+
+    def decode_attention(self, pool, query, kv_heads, seq_lens, max_len, **kw):
+        self.calls.append(("decode", query, seq_lens, kw["block_tables"], kw.get("out")))
+        return kw["out"] if kw.get("out") is not None else torch.zeros_like(query)
+
+    def prefill_attention(self, pool, query, kv_heads, query_start, seq_lens, max_len, block_tables, block_size, **kw):
+        self.calls.append(("prefill", query.shape[0], seq_lens.tolist(), max_len, kw["first_token"]))
+        return kw["out"]
+
+
+def _v1_call(query_lens, seq_lens, pad=0, **extra):
+    """One layer call of the v1 backend on a stand-in store: (calls of the store, metadata)."""
+    v1 = pytest.importorskip("turboquant_kv.vllm_plugin.v1_backend")
+    impl = v1.TurboQuantV1Impl(8, 64, 0.125, 2)
+    impl._kv = _StandInStore()
+    n, reqs, blocks = sum(query_lens), len(query_lens), -(-max(seq_lens) // 16)
+    qsl = torch.tensor([0] + list(np.cumsum(query_lens)), dtype=torch.int32)
+    md = v1.TurboQuantV1Metadata(
+        num_reqs=reqs, num_actual_tokens=n, max_query_len=max(query_lens), max_seq_len=max(seq_lens), query_start_loc=qsl,
+        query_start_loc_cpu=qsl, seq_lens=torch.tensor(seq_lens, dtype=torch.int32),
+        block_table=torch.zeros(reqs, blocks, dtype=torch.int32), slot_mapping=torch.arange(n + pad), **extra)
+    q, k = torch.zeros(n + pad, 8 * 64), torch.zeros(n + pad, 2 * 64)
+    out = impl.forward(None, q, k, k, torch.zeros(4, 2, _StandInStore.record_bytes, dtype=torch.uint8), md, output=torch.empty_like(q))
+    assert out.shape == q.shape
+    return impl._kv.calls, md
+
+
+def test_v1_decode_batch_is_handed_over_whole():
+    """A pure decode batch passes the metadata's tensors as they are (a small call is bound by the host); a mixed one is split."""
+    calls, md = _v1_call([1, 1, 1], [40, 7, 90])
+    assert [c[0] for c in calls] == ["append", "decode"]
+    assert calls[1][2] is md.seq_lens and calls[1][3] is md.block_table and calls[1][1].shape == (3, 8, 64)
+    calls, md = _v1_call([1, 1], [40, 7], pad=3)                # rows behind the batch's tokens are padding
+    assert calls[1][2] is md.seq_lens and calls[1][1].shape[0] == 2
+    calls, md = _v1_call([1, 1, 30], [40, 7, 90])
+    assert [c[0] for c in calls] == ["append", "decode", "prefill"]
+    assert calls[1][1].shape[0] == 2 and calls[1][2].tolist() == [40, 7] and calls[2][1:] == (30, [90], 90, 2)
+
+
 def test_attention_function_registers_with_transformers_and_defaults_to_the_library_path():
     """Without an attached cache the registered attention function is transformers' own SDPA call."""
     pytest.importorskip("transformers")
