@@ -206,9 +206,9 @@ int tqb_kv_update(uint8_t* store, int64_t batch, int64_t heads, int64_t unit_pit
  *
  * workspace: device scratch of at least tqb_decode_attention_workspace_bytes(...) bytes, 256-byte
  * aligned, not shared between calls that may overlap on the device.  The caller ZEROES it once before
- * its first use (cudaMemsetAsync); after that the kernel keeps its counters clean by itself.  Its first
- * 4 bytes are a status word in which the kernel only ever SETS bits (TQB_DECODE_* below); the caller
- * reads and clears it.  After TQB_DECODE_WAIT_EXPIRED or TQB_DECODE_NO_SMEM the results of that call
+ * its first use (cudaMemsetAsync); after that the kernel keeps its counters clean by itself, also between
+ * calls of different batch sizes, lengths and heads.  Its first 4 bytes are a status word in which the kernel
+ * only ever SETS bits (TQB_DECODE_* below); the caller reads and clears it.  After TQB_DECODE_WAIT_EXPIRED or TQB_DECODE_NO_SMEM the results of that call
  * are invalid and the whole workspace must be zeroed again before the next call.
  *
  * Lengths are clamped on the device: a seq_lens[b] that is negative or exceeds max_len (a stale host

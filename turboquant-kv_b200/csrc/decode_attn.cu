@@ -59,6 +59,10 @@ constexpr int LEN_ROOM = 1 << 30;       // flag in an encoded length: this step 
 constexpr int LEN_MASK = LEN_ROOM - 1;
 constexpr int64_t MAX_LEN_LIMIT = (int64_t)1 << 30;
 constexpr int MERGE_MAX_CHUNKS = 1024;  // partials per (unit, query head) the planner allows
+// Arrival counters come first in the workspace and have this much of it to themselves whatever the batch: one workspace
+// serves calls of any batch, and no call may leave its partials where a call of more units counts arrivals.  Calls of more
+// units than that zero their counters themselves.
+constexpr size_t COUNTER_BYTES = 64 * 1024;
 
 // ---- launch parameters --------------------------------------------------------------------------
 struct DecodeParams {
@@ -1259,7 +1263,7 @@ static DecodeWorkspace plan_workspace(int batch, int q_heads, int kv_heads, int 
     w.flat = batch <= 256 && max_tiles + sm_count() < 0x7fffffff && flat_cost < 0.98 * chunk_cost;
     size_t off = 0;
     w.off_status = off; off = align_up(off + 256, 256);                    // status word, exit counter
-    w.off_cnt = off;    off = align_up(off + (size_t)units * 4, 256);      // arrival counter per unit
+    w.off_cnt = off;    off = align_up(off + std::max(COUNTER_BYTES, (size_t)units * 4), 256);      // arrival counter per unit
     // partial slots: one per (unit, chunk), or one per (unit, CTA that streams a piece of it): slot = CTA + unit
     const size_t slots = w.flat ? (size_t)units + sm_count() : (size_t)units * w.nchunks;
     const size_t parts = slots * sets * group;
@@ -1370,6 +1374,8 @@ static int decode_common(const void* query, int q_dtype, const void* key, const 
     p.part_l = reinterpret_cast<float*>(ws + w.off_l);
     p.part_acc = reinterpret_cast<float*>(ws + w.off_acc);
     cudaStream_t st = (cudaStream_t)stream;
+    const size_t counters = (size_t)batch * kv_heads * sizeof(int);
+    if (counters > COUNTER_BYTES) TQB_CUDA(cudaMemsetAsync(p.unit_cnt, 0, counters, st));
     if (dim == 64) return paged ? dispatch_bits<64, true>(kbits, vbits, p, st) : dispatch_bits<64, false>(kbits, vbits, p, st);
     return paged ? dispatch_bits<128, true>(kbits, vbits, p, st) : dispatch_bits<128, false>(kbits, vbits, p, st);
 }
