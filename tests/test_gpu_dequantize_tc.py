@@ -137,3 +137,22 @@ def test_cache_update_keeps_the_gradient_of_new_tokens():
     assert ka.shape == (2, 2, 6, 64)
     with torch.no_grad():
         assert not cache.update(k, v, 0)[0].requires_grad
+
+
+@pytest.mark.parametrize("shape", [(1, 2, 1, 64), (2, 1, 1, 64), (2, 2, 3, 32), (3, 2, 1, 64), (2, 5, 1, 64), (2, 2, 1, 128)])
+def test_cache_update_refuses_states_of_another_shape(shape):
+    """A layer's batch, heads and head_dim are those of its first update; nothing is stored when others come."""
+    from turboquant_kv import TurboQuantCache
+
+    cache = TurboQuantCache(key_bits=4, value_bits=2, seed=42)
+    k, v = (torch.randn(2, 2, 5, 64, device="cuda") for _ in range(2))
+    cache.update(k, v, 0)
+    store = cache._layer_stores[0]._store.clone()
+    bad = torch.randn(*shape, device="cuda")
+    with pytest.raises(RuntimeError):
+        cache.update(bad, bad, 0)
+    with pytest.raises(RuntimeError):
+        cache.append_only(bad, bad, 0)
+    with pytest.raises(RuntimeError):
+        cache.update(k, v[:, :, :3], 0)
+    assert cache.get_seq_length(0) == 5 and torch.equal(store, cache._layer_stores[0]._store)

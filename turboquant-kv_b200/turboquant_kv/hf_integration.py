@@ -62,8 +62,14 @@ class _LayerQuantStore:
             new[:, : self._store.shape[1]] = self._store
         self._store, self.capacity = new, cap
 
+    def _check(self, key: torch.Tensor, value: torch.Tensor) -> None:
+        B, H, D = self.batch, self.num_heads, self.head_dim
+        if key.dim() != 4 or value.shape != key.shape or key.shape[:2] != (B, H) or key.shape[3] != D:
+            raise RuntimeError(f"the layer holds ({B}, {H}, tokens, {D}) states, got keys {tuple(key.shape)} and values {tuple(value.shape)}")
+
     def append(self, key: torch.Tensor, value: torch.Tensor) -> None:
         """key / value: (batch, heads, new, head_dim)."""
+        self._check(key, value)
         T = key.shape[2]
         self._reserve(self.seq_len + T)
         rm = N.RowMap(T, self.capacity, 1, self.seq_len, None, 1, None, 1)
@@ -73,9 +79,10 @@ class _LayerQuantStore:
     def update(self, key: torch.Tensor, value: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
         """``append``, and the dense history: (batch, heads, total, head_dim) keys and values in the inputs' dtype, old tokens
         dequantised, new tokens exact."""
+        self._check(key, value)
         dt, T = key.dtype, key.shape[2]
         if (dt in (torch.float32, torch.float16, torch.bfloat16) and value.dtype == dt and key.device == self.device
-                and value.device == self.device and key.stride(3) == 1 and value.stride(3) == 1 and value.shape == key.shape):
+                and value.device == self.device and key.stride(3) == 1 and value.stride(3) == 1):
             self._reserve(self.seq_len + T)
             out = self.kv.update(self._store, self.capacity, self.seq_len, key, value)
             self.seq_len += T
