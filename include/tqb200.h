@@ -180,7 +180,8 @@ int tqb_kv_dequantize(const uint8_t* store, int64_t units, int64_t unit_pitch, i
 /* One cache update under the dense contract of TurboQuantCache.update (turboquant_kv/hf_integration.py:340-390): k_out /
  * v_out (batch, heads, old_tokens + new_tokens, dim) receive the old tokens dequantised and the new tokens as they are, and
  * the new tokens are quantised into positions old_tokens .. of their units.  key / value (batch, heads, new_tokens, dim) of
- * `dtype` with unit stride along dim; the strides arrays give the elements between batch items, heads and tokens. */
+ * `dtype` with unit stride along dim; the strides arrays give the elements between batch items, heads and tokens.  Several
+ * new tokens behind old ones are stored by one launch where key and value are contiguous, else by one per unit. */
 int tqb_kv_update(uint8_t* store, int64_t batch, int64_t heads, int64_t unit_pitch, int64_t old_tokens, int64_t new_tokens,
                   int dim, const void* key, const int64_t* key_strides, const void* value, const int64_t* value_strides,
                   int dtype, const float* rot_k, const float* bnd_k, const float* cent_k, int kbits, const float* rot_v,

@@ -156,3 +156,21 @@ def test_cache_update_refuses_states_of_another_shape(shape):
     with pytest.raises(RuntimeError):
         cache.update(k, v[:, :, :3], 0)
     assert cache.get_seq_length(0) == 5 and torch.equal(store, cache._layer_stores[0]._store)
+
+
+def test_update_of_several_tokens_costs_the_same_launches_for_any_batch():
+    """Several tokens behind old ones are stored by one append over all sequences and heads, however the states are laid out."""
+    from turboquant_kv import TurboQuantCache, _native as N
+
+    counts = []
+    for batch, heads in ((1, 1), (8, 8)):
+        for layout in ("bhtd", "bthd"):
+            cache = TurboQuantCache(key_bits=4, value_bits=2, seed=42)
+            for T in (300, 30):
+                k, v = (torch.randn(batch, heads, T, 64, device="cuda") for _ in range(2))
+                if layout == "bthd":
+                    k, v = (t.transpose(1, 2).contiguous().transpose(1, 2) for t in (k, v))
+                before = N.launch_count()
+                cache.update(k, v, 0)
+            counts.append(N.launch_count() - before)
+    assert len(set(counts)) == 1, counts

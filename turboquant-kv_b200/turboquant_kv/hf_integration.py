@@ -84,6 +84,8 @@ class _LayerQuantStore:
         if (dt in (torch.float32, torch.float16, torch.bfloat16) and value.dtype == dt and key.device == self.device
                 and value.device == self.device and key.stride(3) == 1 and value.stride(3) == 1):
             self._reserve(self.seq_len + T)
+            if T > 1 and self.seq_len:                   # (one append for all sequences and heads wants packed rows)
+                key, value = key.contiguous(), value.contiguous()
             out = self.kv.update(self._store, self.capacity, self.seq_len, key, value)
             self.seq_len += T
             return out
