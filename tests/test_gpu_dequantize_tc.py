@@ -174,3 +174,21 @@ def test_update_of_several_tokens_costs_the_same_launches_for_any_batch():
                 cache.update(k, v, 0)
             counts.append(N.launch_count() - before)
     assert len(set(counts)) == 1, counts
+
+
+def test_cache_update_keeps_the_tangent_of_new_tokens():
+    """Forward-mode derivatives pass through the dense history as gradients do."""
+    import torch.autograd.forward_ad as fwad
+
+    from turboquant_kv import TurboQuantCache
+
+    cache = TurboQuantCache(key_bits=4, value_bits=2, seed=42)
+    for T in (5, 1, 3):
+        old = cache.get_seq_length(0)
+        k, v, dk, dv = (torch.randn(2, 2, T, 64, device="cuda") for _ in range(4))
+        with fwad.dual_level(), torch.no_grad():
+            ka, va = cache.update(fwad.make_dual(k, dk), fwad.make_dual(v, dv), 0)
+            (ka, ta), (va, tv) = fwad.unpack_dual(ka), fwad.unpack_dual(va)
+            assert ta is not None and tv is not None
+            assert torch.equal(ta[:, :, old:], dk) and torch.equal(tv[:, :, old:], dv) and not ta[:, :, :old].any()
+        assert torch.equal(ka[:, :, old:], k) and ka.shape[2] == old + T

@@ -21,6 +21,7 @@ import weakref
 from typing import Any, Dict, List, Optional, Tuple
 
 import torch
+from torch.autograd.forward_ad import unpack_dual
 
 from . import _native as N
 from .config import TurboQuantConfig
@@ -35,6 +36,11 @@ try:
     _TRANSFORMERS_AVAILABLE = True
 except ImportError:  # pragma: no cover
     pass
+
+
+def _differentiated(*states: torch.Tensor) -> bool:
+    """Whether a gradient (reverse mode) or a tangent (forward mode) flows through the states."""
+    return any((t.requires_grad and torch.is_grad_enabled()) or unpack_dual(t).tangent is not None for t in states)
 
 
 class _LayerQuantStore:
@@ -266,8 +272,8 @@ class TurboQuantCache(_DynamicCache):  # type: ignore[misc]
             # the attention function registered by attach() reads the packed records itself
             st.append(key_states, value_states)
             return key_states, value_states
-        if isinstance(st, _LayerQuantStore) and not (torch.is_grad_enabled() and (key_states.requires_grad or value_states.requires_grad)):
-            return st.update(key_states, value_states)     # (gradients of the new tokens go through the concatenation below)
+        if isinstance(st, _LayerQuantStore) and not _differentiated(key_states, value_states):
+            return st.update(key_states, value_states)     # (derivatives of the new tokens go through the concatenation below)
         dt = key_states.dtype if key_states.dtype in (torch.float16, torch.bfloat16) else torch.float32
         k_old, v_old = st.get_keys(dt), st.get_values(dt)
         st.append(key_states, value_states)
