@@ -37,6 +37,30 @@ def test_host_constants_match_upstream(golden):
         R.make_rotation_matrix(8, 1, "nope")
 
 
+def test_rotation_seeds_that_name_no_matrix_are_not_remembered():
+    """Repeated calls share the factorisation of an integer seed only; results are the caller's own."""
+    import turboquant_kv.reference as R
+
+    a, b = R.make_rotation_matrix(32, 7), R.make_rotation_matrix(32, 7)
+    assert torch.equal(a, b)
+    a.zero_()
+    assert torch.equal(R.make_rotation_matrix(32, 7), b) and torch.equal(R.make_rotation_matrix(32, np.int64(7)), b)
+    assert not torch.equal(R.make_rotation_matrix(16, None), R.make_rotation_matrix(16, None))
+    assert torch.equal(R.make_rotation_matrix(16, [1, 2]), R.make_rotation_matrix(16, np.array([1, 2])))
+    R.make_rotation_matrix(16, 3)
+    with pytest.raises(TypeError):
+        R.make_rotation_matrix(16, 3.0)
+    default = torch.get_default_dtype()
+    want = R.make_rotation_matrix(24, 5, "rht")
+    try:                                                    # the Hadamard construction follows torch's default type
+        torch.set_default_dtype(torch.float64)
+        assert R.make_rotation_matrix(24, 5, "rht").dtype == torch.float32
+        assert torch.equal(R.make_rotation_matrix(24, 5, "rht"), R.make_rht_rotation(24, 5))
+    finally:
+        torch.set_default_dtype(default)
+    assert torch.equal(R.make_rotation_matrix(24, 5, "rht"), want)
+
+
 def test_codebook_properties():
     """What upstream tests/test_reference.py checks of the codebook: analytic 1-bit value, counts, order, symmetry."""
     import turboquant_kv.reference as R

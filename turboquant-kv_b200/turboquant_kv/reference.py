@@ -72,21 +72,23 @@ def lloyd_max_codebook(bits: int, dim: int) -> Tuple[torch.Tensor, torch.Tensor]
 
 def make_rotation_matrix(dim: int, seed: int = 42, method: str = "dense_qr") -> torch.Tensor:
     """Random orthogonal (dim, dim) float32 matrix: "dense_qr" (paper) or "rht" (Hadamard based)."""
-    return _rotation_matrix(dim, seed, method).clone()
-
-
-@lru_cache(maxsize=64)
-def _rotation_matrix(dim: int, seed: int, method: str) -> torch.Tensor:
-    # (a factorisation takes milliseconds on the host, and every layer of every cache asks for the same few)
     if method == "dense_qr":
-        gauss = np.random.RandomState(seed).randn(dim, dim).astype(np.float32)
-        q, r = np.linalg.qr(gauss)
-        flip = np.sign(np.diag(r))
-        flip[flip == 0] = 1.0  # keeps Q unique: diag(R) > 0
-        return torch.from_numpy(np.ascontiguousarray(q * flip[None, :]))
+        # (only a plain integer names one matrix: a seed of None draws another every time, arrays cannot be looked up, 42.0 is refused)
+        make = _dense_qr if type(dim) is int and type(seed) is int else _dense_qr.__wrapped__
+        return torch.from_numpy(make(dim, seed).copy())
     if method == "rht":
         return make_rht_rotation(dim, seed)
     raise ValueError(f"Unknown rotation method: {method}")
+
+
+@lru_cache(maxsize=64)
+def _dense_qr(dim: int, seed: int) -> np.ndarray:
+    # (a factorisation takes milliseconds on the host, and every layer of every cache asks for the same few)
+    gauss = np.random.RandomState(seed).randn(dim, dim).astype(np.float32)
+    q, r = np.linalg.qr(gauss)
+    flip = np.sign(np.diag(r))
+    flip[flip == 0] = 1.0  # keeps Q unique: diag(R) > 0
+    return np.ascontiguousarray(q * flip[None, :])
 
 
 def make_rht_rotation(dim: int, seed: int = 42) -> torch.Tensor:
