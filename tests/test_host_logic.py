@@ -281,6 +281,30 @@ def test_v1_decode_batch_is_handed_over_whole():
     assert calls[1][1].shape[0] == 2 and calls[1][2].tolist() == [40, 7] and calls[2][1:] == (30, [90], 90, 2)
 
 
+def test_v1_few_token_rule_looks_at_the_requests_it_serves():
+    """Short prompts beside a long decode take the prefill kernel where the host knows the lengths; few tokens behind a long
+    context of their own take the decode kernel, token by token."""
+    lens = torch.tensor([20_000, 30, 25], dtype=torch.int32)
+    calls, _ = _v1_call([1, 30, 25], lens.tolist(), seq_lens_cpu=lens)
+    assert [c[0] for c in calls] == ["append", "decode", "prefill"] and calls[2][2] == [30, 25]
+    calls, _ = _v1_call([1, 30, 25], lens.tolist())             # lengths on the device only: the batch's bound
+    assert [c[0] for c in calls] == ["append", "decode", "decode"]
+    lens = torch.tensor([20_000, 9000, 25], dtype=torch.int32)
+    calls, _ = _v1_call([1, 5, 25], lens.tolist(), seq_lens_cpu=lens)
+    assert [c[0] for c in calls] == ["append", "decode", "decode"]
+    calls, _ = _v1_call([8], [7000], seq_lens_cpu=torch.tensor([7000]))
+    assert [c[0] for c in calls] == ["append", "decode"]
+    v1 = pytest.importorskip("turboquant_kv.vllm_plugin.v1_backend")
+    from vllm.v1.attention.backend import CommonAttentionMetadata
+
+    qsl, lens = torch.tensor([0, 3], dtype=torch.int32), torch.tensor([9], dtype=torch.int32)
+    common = CommonAttentionMetadata(query_start_loc=qsl, query_start_loc_cpu=qsl, seq_lens=lens, num_reqs=1, num_actual_tokens=3, max_query_len=3,
+                                     max_seq_len=9, block_table_tensor=torch.zeros(1, 1, dtype=torch.int32), slot_mapping=torch.arange(3),
+                                     seq_lens_cpu_upper_bound=lens)
+    md = v1.TurboQuantV1MetadataBuilder(None, ["l0"], None, "cpu").build(0, common)
+    assert md.seq_lens_cpu is lens
+
+
 def test_attention_function_registers_with_transformers_and_defaults_to_the_library_path():
     """Without an attached cache the registered attention function is transformers' own SDPA call."""
     pytest.importorskip("transformers")

@@ -105,6 +105,7 @@ class TurboQuantV1Metadata:
     block_table: torch.Tensor              # (num_reqs, max_blocks) int32, device
     slot_mapping: torch.Tensor             # (num_tokens,) int64, device; negative = padding
     causal: bool = True
+    seq_lens_cpu: Optional[torch.Tensor] = None    # the lengths (or upper bounds of them) on the host, where the engine has them
 
 
 class TurboQuantV1MetadataBuilder(AttentionMetadataBuilder[TurboQuantV1Metadata]):
@@ -117,10 +118,14 @@ class TurboQuantV1MetadataBuilder(AttentionMetadataBuilder[TurboQuantV1Metadata]
     def build(self, common_prefix_len: int, common_attn_metadata: CommonAttentionMetadata,
               fast_build: bool = False) -> TurboQuantV1Metadata:
         m = common_attn_metadata
+        host = getattr(m, "_seq_lens_cpu", None)           # (the property of that name would wait for the device)
+        if host is None:
+            host = getattr(m, "seq_lens_cpu_upper_bound", None)
         return TurboQuantV1Metadata(
             num_reqs=m.num_reqs, num_actual_tokens=m.num_actual_tokens, max_query_len=m.max_query_len,
             max_seq_len=m.max_seq_len, query_start_loc=m.query_start_loc, query_start_loc_cpu=m.query_start_loc_cpu,
-            seq_lens=m.seq_lens, block_table=m.block_table_tensor, slot_mapping=m.slot_mapping, causal=m.causal)
+            seq_lens=m.seq_lens, block_table=m.block_table_tensor, slot_mapping=m.slot_mapping, causal=m.causal,
+            seq_lens_cpu=host)
 
 
 class TurboQuantV1Impl(AttentionImpl[TurboQuantV1Metadata]):
@@ -200,7 +205,10 @@ class TurboQuantV1Impl(AttentionImpl[TurboQuantV1Metadata]):
 
         # 2b. requests with several new tokens
         reqs = md.num_reqs - lead
-        if not self._few_tokens(n - lead, HK, md.max_seq_len):
+        longest = md.max_seq_len                           # of these requests, where the host knows: not of the decodes before them
+        if lead and md.seq_lens_cpu is not None:
+            longest = min(longest, int(md.seq_lens_cpu[lead:md.num_reqs].max()))
+        if not self._few_tokens(n - lead, HK, longest):
             qsl = md.query_start_loc[lead:md.num_reqs + 1].to(torch.int32).contiguous()
             kv.prefill_attention(pool, q[lead:], HK, qsl, lens[lead:md.num_reqs], md.max_seq_len, bt[lead:], block_size,
                                  causal=md.causal, scale=self.scale, out=out[lead:], first_token=lead)
