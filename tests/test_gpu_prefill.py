@@ -105,6 +105,21 @@ def test_prefill_attention_many_items_long_context_and_clamped_lengths(orc):
     assert not none.any()
 
 
+def test_prefill_takes_queries_of_other_types():
+    """A float64 query computes in float32, into an output of its own type, as decode queries do."""
+    from turboquant_kv.kvstore import PackedKVStore
+
+    dev, dim, kvh, bs = torch.device("cuda"), 64, 2, 16
+    kv = PackedKVStore(dim, 4, 2, 42, "dense_qr", dev)
+    pool, tables, _ = _pool(kv, [50], kvh, dim, bs, torch.float32, seed=3)
+    q = torch.randn(20, 4, dim, generator=torch.Generator().manual_seed(1)).cuda()
+    args = (kvh, torch.tensor([0, 20], dtype=torch.int32, device=dev), torch.tensor([50], dtype=torch.int32, device=dev), 50, tables, bs)
+    want = kv.prefill_attention(pool, q, *args)
+    out = torch.empty(20, 4, dim, dtype=torch.float64, device=dev)
+    assert kv.prefill_attention(pool, q.double(), *args, out=out) is out and torch.equal(out, want.double())
+    assert torch.equal(kv.prefill_attention(pool, q.double().cpu(), *args), want)
+
+
 def test_v1_mixed_batch_splits_decodes_and_prefills(orc):
     """Decodes at the head go to the decode kernel, the rest to the prefill kernel, a one-token request behind them too; the
     outcome is that of a batch in another order."""

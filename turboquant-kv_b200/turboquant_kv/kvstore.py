@@ -195,12 +195,16 @@ class PackedKVStore:
     def prefill_attention(self, store: torch.Tensor, query: torch.Tensor, kv_heads: int, query_start: torch.Tensor,
                           seq_lens: torch.Tensor, max_len: int, block_tables: torch.Tensor, block_size: int, causal: bool = True,
                           scale: Optional[float] = None, out: Optional[torch.Tensor] = None, first_token: int = 0) -> torch.Tensor:
-        """query (tokens, q_heads, head_dim), several tokens per request, over a paged pool -> the same shape and dtype.
+        """query (tokens, q_heads, head_dim), several tokens per request, over a paged pool -> the same shape in the query's dtype
+        (float32 for a dtype that the kernels do not take), or in ``out``.
 
         ``query_start`` (requests + 1,) and ``seq_lens`` (requests,) are device int32: a request's tokens are the last of its
         ``seq_lens`` tokens, all stored already.  ``query_start`` counts from ``first_token``, the query's first row.  ``max_len``
         bounds ``seq_lens``."""
-        q = query.contiguous()
+        q = query.to(self.device)
+        if q.dtype not in (torch.float32, torch.float16, torch.bfloat16):
+            q = q.float()
+        q = q.contiguous()
         if q.data_ptr() % 16:
             q = q.clone()
         n, HQ, D = q.shape
