@@ -88,3 +88,35 @@ def test_few_tokens_behind_a_long_decode_in_one_batch(orc):
                 attention_close(out[i:i + 1].view(1, kvh * group, dim).float().cpu().numpy(), ref)
     finally:
         B.configure()
+
+
+def test_status_survives_a_larger_workspace_and_tells_of_every_kernel(monkeypatch):
+    """A clamped prefill call is still reported after a decode call has replaced the workspace by a larger one; an expired wait of
+    the tensor-core kernels that have no workspace is reported too (their word is read through the library: a stand-in here)."""
+    from turboquant_kv import _native as N, reference
+    from turboquant_kv.kvstore import STATUS_LEN_CLAMPED, STATUS_WAIT_EXPIRED, PackedKVStore
+
+    dev, dim, kvh, bs = torch.device("cuda"), 64, 2, 16
+    kv = PackedKVStore(dim, 4, 2, 42, "dense_qr", dev)
+    pool, tables, _ = _pool(kv, [300, 80], kvh, dim, bs, torch.float16, seed=1)
+    lens = torch.tensor([300, 80], dtype=torch.int32, device=dev)
+    q = torch.randn(10, 4, dim, device=dev).half()
+    assert kv.status() == 0
+    kv.prefill_attention(pool, q, kvh, torch.tensor([0, 10], dtype=torch.int32, device=dev), lens[:1].contiguous(), 200, tables[:1], bs)
+    small = kv._workspace
+    kv.decode_attention(pool, q[:2], kvh, lens, 300, block_tables=tables, block_size=bs)
+    assert kv._workspace is not small
+    assert kv.status() == STATUS_LEN_CLAMPED and kv.status() == 0
+    words = [1, 0]
+
+    class Lib:
+        def __getattr__(self, name):
+            return getattr(N._lib, name)
+
+        def tqb_quantize_status(self, stream):
+            return words.pop(0)
+
+    real = N.lib()
+    monkeypatch.setattr(N, "_lib", real, raising=False)
+    monkeypatch.setattr(N, "lib", lambda: Lib())
+    assert kv.status() == STATUS_WAIT_EXPIRED and reference.kernel_status() == 0

@@ -16,7 +16,7 @@ from typing import Optional, Tuple
 import torch
 
 from . import _native as N
-from .reference import lloyd_max_codebook, make_rotation_matrix
+from .reference import kernel_status, lloyd_max_codebook, make_rotation_matrix
 
 
 STATUS_WAIT_EXPIRED, STATUS_NO_SMEM, STATUS_UNIT_FULL, STATUS_LEN_CLAMPED = 1, 2, 4, 8   # TQB_DECODE_* of tqb200.h
@@ -268,17 +268,22 @@ class PackedKVStore:
     def _reserve_workspace(self, need: int) -> None:
         """The decode workspace starts zeroed (status word, arrival counters); the kernel keeps it clean."""
         if self._workspace is None or self._workspace.numel() < need:
-            self._workspace = torch.zeros(need, dtype=torch.uint8, device=self.device)
+            grown = torch.zeros(need, dtype=torch.uint8, device=self.device)
+            if self._workspace is not None:
+                grown[:4] = self._workspace[:4]          # the status that earlier calls have raised
+            self._workspace = grown
 
     def status(self) -> int:
-        """Status bits raised by the decode calls since the last status() (synchronises, then clears them):
+        """Status bits raised by the attention calls since the last status() (synchronises, then clears them):
         0 = all good; STATUS_WAIT_EXPIRED / STATUS_NO_SMEM = results invalid (the workspace is re-zeroed here);
         STATUS_UNIT_FULL = a fused step found a full unit and dropped its token; STATUS_LEN_CLAMPED = a
-        sequence length outside the announced bounds was clamped."""
+        sequence length outside the announced bounds was clamped.  STATUS_WAIT_EXPIRED also tells of an expired wait in the
+        tensor-core kernels of appends, updates and dequantised keys and values on this device (`reference.kernel_status`)."""
+        value = STATUS_WAIT_EXPIRED if kernel_status(self.device) else 0
         if self._workspace is None:
-            return 0
+            return value
         word = self._workspace[:4].view(torch.int32)
-        value = int(word.item())
+        value |= int(word.item())
         if value & (STATUS_WAIT_EXPIRED | STATUS_NO_SMEM):
             self._workspace.zero_()
         elif value:

@@ -117,6 +117,17 @@ def _packed_dim(dim: int, bits: int) -> int:
     return bits * ((dim + 7) // 8)
 
 
+def kernel_status(device=None) -> int:
+    """0, or 1 where a bounded wait of a tensor-core kernel (quantisers, dequantisers, the index scan's ranking pass) has expired
+    on the device since the last call: outputs of the calls since then may be invalid (a search answers from its list kernels
+    instead).  Synchronises the current stream and clears the word."""
+    with torch.cuda.device(device):
+        word = N.lib().tqb_quantize_status(torch.cuda.current_stream().cuda_stream)
+    if word < 0:
+        N.check(word)
+    return int(word != 0)
+
+
 # --------------------------------------------------------------------------------------------
 # pack / unpack
 # --------------------------------------------------------------------------------------------
