@@ -68,3 +68,29 @@ def test_prod_overflow_and_repeated_rows():
         idx.add(torch.from_numpy(np.repeat(row, 100_000, axis=0)))
         scores, ids = idx.search(torch.from_numpy(np.repeat(row, 20, axis=0)), 10)
         assert torch.equal(ids, torch.arange(10).repeat(20, 1)) and bool((scores == scores[0, 0]).all())
+
+
+def test_queries_that_tie_everywhere_stop_gathering():
+    """Zero queries overflow their buffers at once: the pass drops them and the list kernels answer, in about the list kernels' time."""
+    from turboquant_kv import TurboQuantIndex
+
+    db, qs = _data(400_000, 128, 32, seed=8)
+    idx = TurboQuantIndex(dim=128, bit_width=4, seed=42)
+    idx.add(torch.from_numpy(db))
+    q = torch.from_numpy(qs).cuda()
+    zeros = q.clone()
+    zeros[4:] = 0.0
+
+    def best_ms(queries):
+        times = []
+        for _ in range(4):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            idx.search(queries, 10)
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times)
+
+    lists = 4 * best_ms(q[:8])                               # four passes of eight
+    assert best_ms(zeros) < 4 * (lists + best_ms(q))         # (counting all of them took 48 times as long)

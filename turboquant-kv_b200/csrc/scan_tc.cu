@@ -318,6 +318,8 @@ __global__ void __launch_bounds__(ST_THREADS, 1) scan_tc_kernel(const ScanTcArgs
                 if (at < a.cap) {
                     a.buf_s[(int64_t)q * a.cap + at] = __uint_as_float(log[3 * e + 1]);
                     a.buf_i[(int64_t)q * a.cap + at] = (int)log[3 * e + 2];
+                } else {                                   // overflowed: no more of this query's rows (32 queries, 28 of them zero,
+                    thr_s[q - q0] = -ST_NEG_INF;           // over 1 M rows: 17.5 ms where all were counted)
                 }
             }
             __syncwarp();
