@@ -94,3 +94,50 @@ def test_queries_that_tie_everywhere_stop_gathering():
 
     lists = 4 * best_ms(q[:8])                               # four passes of eight
     assert best_ms(zeros) < 4 * (lists + best_ms(q))         # (counting all of them took 48 times as long)
+
+
+def _in_shards(idx, q, k, rows=1000):
+    """The search of a Prod-mode index in shards of so few rows that the float32 list kernel ranks them."""
+    from turboquant_kv import TurboQuantIndex
+    from turboquant_kv.search import merge_topk
+
+    found = []
+    for lo in range(0, idx.n_vectors, rows):
+        part = TurboQuantIndex(dim=idx.dim, bit_width=idx.bit_width, mode="prod", seed=42)
+        for name in ("_packed_codes", "_norms", "_qjl_signs", "_residual_norms"):
+            setattr(part, name, getattr(idx, name)[lo:lo + rows].contiguous())
+        part.n_vectors, part.id_offset = part._norms.shape[0], lo
+        found.append(part.search(q, k))
+    return merge_topk(torch.stack([s for s, _ in found], 1), torch.stack([i for _, i in found], 1), k)
+
+
+@pytest.mark.parametrize("mode,k", [("mse", 10), ("mse", 40), ("prod", 10)])
+def test_rows_and_queries_that_are_not_finite(mode, k):
+    """Infinite norms rank first (or last), NaN rows never; a query that is not finite leaves the others alone.  The same answers
+    as calls of few queries over the same rows, or, in Prod mode, of few rows at a time."""
+    from turboquant_kv import TurboQuantIndex
+
+    n, dim, nq = 24_000, 64, 24
+    db, qs = _data(n, dim, nq, seed=5)
+    qs[5, 3], qs[11, 0], qs[17] = np.nan, np.inf, 0.0
+    idx = TurboQuantIndex(dim=dim, bit_width=3, mode=mode, seed=42)
+    idx.add(torch.from_numpy(db))
+    if mode == "mse":
+        packed, norms = idx._packed_codes.clone(), idx._norms.clone()
+    else:
+        norms = idx._norms
+    norms[17::300] = float("inf")
+    norms[30::500] = float("nan")
+    if mode == "mse":
+        idx._import_rows(packed, norms)
+    q = torch.from_numpy(qs).cuda()
+    scores, ids = idx.search(q, k)
+    if mode == "mse":
+        few = [idx.search(q[i:i + 4], k) for i in range(0, nq, 4)]
+        want_s, want_i = torch.cat([s for s, _ in few]), torch.cat([i for _, i in few])
+    else:
+        want_s, want_i = _in_shards(idx, q, k)
+    assert torch.equal(scores.nan_to_num(7.0), want_s.nan_to_num(7.0))
+    finite = [i for i in range(nq) if i != 17]                  # (a zero query ties everywhere: any k of the rows)
+    assert torch.equal(ids[finite], want_i[finite])
+    assert bool(torch.isinf(scores[0]).all()) and int(ids.max()) < n

@@ -126,9 +126,11 @@ __global__ void __launch_bounds__(256) scan_tc_threshold_kernel(const ScanTcArgs
     }
     __syncthreads();
     if (t == 0) {
-        // the main launch compares unrounded products with it: a little lower, so that the bound's own row stays
-        a.thr[q] = bound - fabsf(bound) * 2e-6f;
-        a.count[q] = 0;
+        // the main launch compares unrounded products with it: a little lower, so that the bound's own row stays (and finite,
+        // so that infinite scores are not below it)
+        a.thr[q] = fminf(bound, 3.4e38f) - fabsf(fminf(bound, 3.4e38f)) * 2e-6f;
+        // the list kernels answer where the sample gave no bound (rows or queries that are not numbers)
+        a.count[q] = bound == ST_NEG_INF ? a.cap + 1 : 0;
     }
 }
 
