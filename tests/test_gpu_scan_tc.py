@@ -141,3 +141,57 @@ def test_rows_and_queries_that_are_not_finite(mode, k):
     finite = [i for i in range(nq) if i != 17]                  # (a zero query ties everywhere: any k of the rows)
     assert torch.equal(ids[finite], want_i[finite])
     assert bool(torch.isinf(scores[0]).all()) and int(ids.max()) < n
+
+
+@pytest.mark.parametrize("dim,k,nq", [(128, 10, 1), (64, 10, 40), (128, 50, 130)])
+def test_prod_rows_that_half_precision_cannot_tell_apart(dim, k, nq):
+    """Rows of one code whose residual norms differ by less than fp16 resolves: the ranking pass sees groups of equal scores, the
+    answer is the float32 order.  Beside them ordinary rows, which most of the queries are near to."""
+    from turboquant_kv import TurboQuantIndex
+
+    n = 30_000
+    gen = torch.Generator().manual_seed(dim + k)
+    rows = torch.randn(n, dim, generator=gen)
+    rows[::10] = rows[7]                                        # 3,000 copies
+    idx = TurboQuantIndex(dim=dim, bit_width=3, mode="prod", seed=42)
+    idx.add(rows)
+    idx._residual_norms[::10] *= 1 + 2e-3 * torch.rand(3000, generator=gen).cuda()
+    q = torch.cat([rows[7][None, :] + 0.3 * torch.randn((nq + 1) // 2, dim, generator=gen), torch.randn(nq // 2, dim, generator=gen)]).cuda()
+    scores, ids = idx.search(q, k)
+    want_s, want_i = _in_shards(idx, q, k)
+    assert torch.equal(scores, want_s) and torch.equal(ids, want_i)
+
+
+@pytest.mark.parametrize("bits,k", [(4, 32), (2, 40), (4, 233), (3, 256)])
+def test_mse_rows_that_half_precision_cannot_tell_apart(bits, k):
+    """Queries whose coordinates differ by less than fp16 resolves, rows that raise one of them each: for k > 24 the ranking keeps
+    22 bits of the queries, whether a call has few or many."""
+    from turboquant_kv import TurboQuantIndex
+    from turboquant_kv import reference as R
+
+    dim, n, raised, nq = 128, 60_000, 6000, 20
+    gen = torch.Generator().manual_seed(bits + k)
+    idx = TurboQuantIndex(dim=dim, bit_width=bits, seed=42)
+    codes = torch.zeros(n, dim, dtype=torch.uint8)
+    where = torch.randperm(n, generator=gen)[:raised]
+    codes[where, torch.arange(raised) % dim] = (1 << bits) - 1
+    idx._import_rows(R.pack_codes(codes.cuda(), bits), torch.ones(n, device="cuda"))
+    idx.n_vectors = n
+    qrot = 1.0 + 2e-4 * torch.rand(nq, dim, generator=gen, dtype=torch.float64)
+    q = (qrot @ idx._rotation.cpu().double()).float()
+    scores, ids = idx.search(q.cuda(), k)
+    few = [idx.search(q[i:i + 4].cuda(), k) for i in range(0, nq, 4)]
+    assert torch.equal(scores, torch.cat([s for s, _ in few])) and torch.equal(ids, torch.cat([i for _, i in few]))
+
+
+@pytest.mark.parametrize("dim,bits,n,nq,k", [(128, 4, 40_003, 16, 233), (64, 3, 90_000, 40, 256), (128, 2, 70_001, 9, 240)])
+def test_the_largest_k(dim, bits, n, nq, k):
+    from turboquant_kv import TurboQuantIndex
+
+    db, qs = _data(n, dim, nq, seed=n + nq)
+    idx = TurboQuantIndex(dim=dim, bit_width=bits, seed=42)
+    idx.add(torch.from_numpy(db))
+    q = torch.from_numpy(qs).cuda()
+    scores, ids = idx.search(q, k)
+    few = [idx.search(q[i:i + 4], k) for i in range(0, nq, 4)]
+    assert torch.equal(scores, torch.cat([s for s, _ in few])) and torch.equal(ids, torch.cat([i for _, i in few]))

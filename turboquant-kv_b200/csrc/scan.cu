@@ -17,12 +17,14 @@
 //                           j = 0..d-1, then * norm), sorts by (score desc, id asc) and emits k.
 // The reported scores are therefore bit-identical to the upstream C++ arithmetic; the tensor-core
 // pass only has to RANK: its scores carry the fp16 rounding of the 16 centroids (relative 2^-12 per
-// term, the queries keep 22 bits).  A true top-k row is lost only if more rows than the margin overtake
-// it through that rounding: 8 within the few thousand rows one warp sees, 24 within the whole database.
+// term) and of the queries (22 bits, or 11 where a pass takes eight queries: calls of more than four with
+// k <= 24).  A true top-k row is lost only if more rows than the margin overtake it through that rounding: 8
+// within the few thousand rows one warp sees, 24 within the whole database.
 //
 // Dims 64 and 128 with 2..4 bits take the tensor-core path; every other supported shape takes
 // scan_generic_kernel (one row per lane, float32 table lookups) with the same list and merge code; so do
-// Prod-mode rows (tqb_scan_topk_prod), with a second term for the QJL sign plane.
+// Prod-mode rows (tqb_scan_topk_prod), with a second term for the QJL sign plane.  Many queries over records, and
+// Prod rows, rank in scan_tc.cu first, and the list kernels then scan only for the queries it leaves to them.
 //
 // scan_records_kernel is the same scan over the key-only records of tiled_layout.cuh (what TurboQuantIndex
 // stores): one table lookup per two codes, one MMA per 16 dims on the centroids' fp16 values, and eight
@@ -33,6 +35,7 @@
 #include "decode_bits.cuh"
 #include "pipe.cuh"
 #include "scan_tc.cuh"
+#include "tc.cuh"
 #include "tiled_layout.cuh"
 
 #include <cmath>
@@ -102,7 +105,10 @@ struct ScanParams {
     float* cand_s; int* cand_id;        // (nq, lists_per_query, kk)
     // After the tensor-core pass (scan_tc.cu): buf_n[q] candidates of query q at buf_*[q * buf_cap]; a query with more than
     // buf_cap of them has overflowed, and only then the list kernels scan for it.  Null: the list kernels scan for all.
-    const int* buf_n; const float* buf_s; const int* buf_i; int buf_cap;
+    int* buf_n; const float* buf_s; const int* buf_i; int buf_cap;
+    // Selections to be proven (scan_tc.cuh): the buffers are merged before the list kernels run, and a query whose selection
+    // cannot be proven is marked as overflowed.  buf_thr: every row not below it is in the buffer.
+    int proven; const float* buf_thr; const uint32_t* buf_limits; const float2* buf_qsum;
     float* out_scores; int64_t* out_ids;
 };
 
@@ -896,6 +902,7 @@ __global__ void __launch_bounds__(SCAN_WARPS * 32) scan_generic_kernel(const Sca
 constexpr int MERGE_THREADS = 256;
 constexpr int MERGE_MAX = TQB_SCAN_MAX_K + SCAN_SELECT_MARGIN + SCAN_TILE;   // selected + tail rows
 constexpr int SURV_MAX = 1024;          // candidates the fast selection path ranks among themselves
+constexpr int PROVEN_MAX = 1024;        // candidates a proven selection re-scores at most
 
 // BUF: after the tensor-core pass (a build of its own: the list merge of a short call is 2 us slower with both inside).
 template <bool BUF>
@@ -903,8 +910,8 @@ __global__ void __launch_bounds__(MERGE_THREADS) scan_merge_kernel(const ScanPar
     extern __shared__ __align__(128) uint8_t smem_raw[];
     const int levels = 1 << p.bits, bpp = (p.dim + 7) >> 3, pd = p.bits * bpp;
     float* T = reinterpret_cast<float*>(smem_raw);     // dim * levels
-    __shared__ float sel_s[MERGE_MAX];
-    __shared__ int sel_i[MERGE_MAX];
+    __shared__ float sel_s[BUF ? PROVEN_MAX + SCAN_TILE : MERGE_MAX];
+    __shared__ int sel_i[BUF ? PROVEN_MAX + SCAN_TILE : MERGE_MAX];
     __shared__ float red_s[MERGE_THREADS / 32];
     __shared__ int red_i[MERGE_THREADS / 32];
     __shared__ float cur_s;
@@ -912,6 +919,8 @@ __global__ void __launch_bounds__(MERGE_THREADS) scan_merge_kernel(const ScanPar
     const int q = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     pdl_trigger();
     pdl_wait();
+    // proven selections: buffers first, then, after the list kernels, the queries that these answered
+    if (p.proven && (p.buf_n[q] <= p.buf_cap) != BUF) return;
     for (int e = tid; e < p.dim * levels; e += blockDim.x)
         T[e] = __fmul_rn(p.qrot[(int64_t)q * p.dim + e / levels], p.cent[e % levels]);
     const bool buffered = BUF && p.buf_n[q] <= p.buf_cap;            // else lists
@@ -926,8 +935,9 @@ __global__ void __launch_bounds__(MERGE_THREADS) scan_merge_kernel(const ScanPar
     __shared__ float sv_s[SURV_MAX];
     __shared__ int sv_i[SURV_MAX];
     __shared__ int surv_n;
-    __shared__ float tau_s;
+    __shared__ float tau_s, kth_s, last_s;      // kth_s, last_s: k-th and ksel-th best of the selection by the scan's scores
     __shared__ int tau_i;
+    if (BUF && tid == 0) { kth_s = -__builtin_huge_valf(); last_s = -__builtin_huge_valf(); }
     if (tid == 0) { surv_n = 0; tau_s = -__builtin_huge_valf(); tau_i = ID_NONE; }
     __syncthreads();
     const int L = p.lists_per_query;
@@ -986,6 +996,8 @@ __global__ void __launch_bounds__(MERGE_THREADS) scan_merge_kernel(const ScanPar
             int rank = 0;
             for (int o = 0; o < surv_n; o++) rank += better(sv_s[o], sv_i[o], sv_s[e], sv_i[e]) ? 1 : 0;
             if (rank < ksel) sel_i[rank] = sv_i[e];
+            if (BUF && rank == p.k - 1) kth_s = sv_s[e];
+            if (BUF && rank == ksel - 1) last_s = sv_s[e];
         }
         __syncthreads();
     }
@@ -1013,11 +1025,38 @@ __global__ void __launch_bounds__(MERGE_THREADS) scan_merge_kernel(const ScanPar
                 if (better(red_s[w], red_i[w], bs, bi)) { bs = red_s[w]; bi = red_i[w]; }
             cur_s = bs; cur_i = bi;
             if (bi != ID_NONE) { sel_i[r] = bi; }
+            if (BUF && bi != ID_NONE && r == p.k - 1) kth_s = bs;
+            if (BUF && bi != ID_NONE && r == ksel - 1) last_s = bs;
         }
         __syncthreads();
         prev_s = cur_s; prev_i = cur_i;
         if (prev_i == ID_NONE) break;
         nsel = r + 1;
+    }
+    if constexpr (BUF) {
+        if (p.proven) {
+            // Nothing below the k-th best by more than twice the scores' error is among the best k: everything above that is
+            // re-scored.  Where the buffer ends before, or holds too many such rows, the list kernels answer.
+            float cmax = 0.0f;
+            for (int c = 0; c < levels; c++) cmax = fmaxf(cmax, fabsf(p.cent[c]));
+            cmax *= fp16_scale(cmax);
+            const float lim = fminf(last_s, kth_s - 2.0f * scan_tc_error(p.buf_limits, p.buf_qsum[q], cmax, p.dim));
+            __syncthreads();
+            if (tid == 0) surv_n = 0;
+            __syncthreads();
+            if (lim >= p.buf_thr[q])                       // (not a number: no proof)
+                for (int64_t e = tid; e < ncand; e += blockDim.x)
+                    if (cs[e] >= lim) {
+                        const int pos = atomicAdd(&surv_n, 1);
+                        if (pos < PROVEN_MAX) sel_i[pos] = ci[e];
+                    }
+            __syncthreads();
+            nsel = surv_n;
+            if (nsel == 0 || nsel > PROVEN_MAX) {
+                if (tid == 0) p.buf_n[q] = p.buf_cap + 1;
+                return;
+            }
+        }
     }
     // ---- tail rows (n % 16) always take part ----
     const int tail = (int)(p.n % SCAN_TILE);
@@ -1116,11 +1155,21 @@ __global__ void topk_merge_kernel(const float* __restrict__ scores, const int64_
     }
 }
 
-static int launch_merge(const ScanParams& p, size_t smem, int pdl, cudaStream_t st) {
-    auto kern = p.buf_n ? scan_merge_kernel<true> : scan_merge_kernel<false>;
+// `buffers`: the merge after the tensor-core pass.
+static int launch_merge(const ScanParams& p, bool buffers, size_t smem, int pdl, cudaStream_t st) {
+    auto kern = buffers ? scan_merge_kernel<true> : scan_merge_kernel<false>;
     TQB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(smem, 48 * 1024)));
     TQB_CUDA(launch_pdl(pdl, kern, dim3(p.nq), dim3(MERGE_THREADS), smem, st, p));
     return check_launch("scan_merge");
+}
+
+// Views of the tensor-core pass's results in its workspace.
+static void take_buffers(ScanParams& p, const ScanTcPlan& t, uint8_t* ws, bool proven) {
+    p.buf_n = reinterpret_cast<int*>(ws + t.off_count); p.buf_cap = t.cap;
+    p.buf_s = reinterpret_cast<const float*>(ws + t.off_s); p.buf_i = reinterpret_cast<const int*>(ws + t.off_i);
+    p.proven = proven ? 1 : 0;
+    p.buf_thr = reinterpret_cast<const float*>(ws + t.off_thr); p.buf_limits = reinterpret_cast<const uint32_t*>(ws + t.off_limits);
+    p.buf_qsum = reinterpret_cast<const float2*>(ws + t.off_qsum);
 }
 
 struct ScanPlan {
@@ -1248,7 +1297,7 @@ static int launch_scan_records(const ScanParams& p, int ngroups, int grid_x, cud
 
 extern "C" size_t tqb_scan_records_workspace_bytes(int nq, int dim, int bits, int k) {
     if (nq <= 0 || (dim != 64 && dim != 128) || bits < 2 || bits > 4 || k <= 0 || k > TQB_SCAN_MAX_K) return 0;
-    return tqb::plan_scan_records(nq, dim, bits, k).total + tqb::scan_tc_plan(nq, dim, false, k, k + tqb::SCAN_SELECT_MARGIN).total;
+    return tqb::plan_scan_records(nq, dim, bits, k).total + tqb::scan_tc_plan(nq, dim, false, k + tqb::SCAN_SELECT_MARGIN).total;
 }
 
 extern "C" int tqb_scan_records_ctas_per_group(int groups, int64_t n, int sms) {
@@ -1274,7 +1323,7 @@ extern "C" int tqb_scan_records_topk(const float* queries, int nq, const uint8_t
     TQB_REQUIRE((uintptr_t)workspace % 256 == 0, "scan_records_topk: workspace must be 256-byte aligned");
     const ScanPlan pl = plan_scan_records(nq, dim, bits, k);
     const int ksel = k + SCAN_SELECT_MARGIN;
-    const ScanTcPlan tpl = scan_tc_plan(nq, dim, false, k, ksel);
+    const ScanTcPlan tpl = scan_tc_plan(nq, dim, false, ksel);
     if (workspace_bytes < pl.total + tpl.total)
         return fail(TQB_ERR_WORKSPACE, "scan_records_topk: workspace %zu bytes < required %zu", workspace_bytes, pl.total + tpl.total);
 
@@ -1300,21 +1349,24 @@ extern "C" int tqb_scan_records_topk(const float* queries, int nq, const uint8_t
     else
         scan_prepare_kernel<QG><<<pl.ngroups, 128, sizeof(float) * (size_t)(1 + 2 * QG) * dim, st>>>(p, 2);
     if (int e = check_launch("scan_prepare")) return e;
-    if (scan_tc_wanted(nq, n - n % SCAN_TILE, dim, bits, false, ksel)) {
+    const size_t msmem = sizeof(float) * (size_t)dim * (1 << bits);
+    // (selections are proven where the list kernels' queries keep 22 bits)
+    const bool proven = rec_queries_per_pass(pl.kk, nq) != RQ;
+    if (scan_tc_wanted(nq, n - n % SCAN_TILE, dim, bits, false, ksel, proven)) {
         ScanTcArgs t{};
         t.records = records; t.rec_bytes = tl_record_bytes(dim, bits, 0); t.rows = n - n % SCAN_TILE; t.dim = dim; t.bits = bits; t.nq = nq;
-        t.k = k; t.ksel = ksel; t.cent = centroids; t.qrot = p.qrot;
+        t.ksel = ksel; t.cent = centroids; t.qrot = p.qrot; t.proven = proven;
         if (int e = scan_tc_run(t, tpl, ws + pl.total, st)) return e;
-        p.buf_n = reinterpret_cast<const int*>(ws + pl.total + tpl.off_count); p.buf_cap = tpl.cap;
-        p.buf_s = reinterpret_cast<const float*>(ws + pl.total + tpl.off_s); p.buf_i = reinterpret_cast<const int*>(ws + pl.total + tpl.off_i);
+        take_buffers(p, tpl, ws + pl.total, proven);
+        if (proven)
+            if (int e = launch_merge(p, true, msmem, 0, st)) return e;
     }
     int e = TQB_ERR_UNSUPPORTED;
 #define TQB_CASE(d, b) if (dim == d && bits == b) e = launch_scan_records<d, b>(p, pl.ngroups, grid_x, st);
     TQB_CASE(64, 2) TQB_CASE(64, 3) TQB_CASE(64, 4) TQB_CASE(128, 2) TQB_CASE(128, 3) TQB_CASE(128, 4)
 #undef TQB_CASE
     if (e) return e;
-    const size_t msmem = sizeof(float) * (size_t)dim * (1 << bits);
-    return launch_merge(p, msmem, 1, st);
+    return launch_merge(p, p.buf_n && !p.proven, msmem, 1, st);
 }
 
 extern "C" size_t tqb_scan_topk_workspace_bytes(int nq, int64_t n, int dim, int bits, int k) {
@@ -1377,14 +1429,14 @@ extern "C" int tqb_scan_topk(const float* queries, int nq, const uint8_t* packed
         if (int e = check_launch("scan_generic")) return e;
     }
     const size_t msmem = sizeof(float) * (size_t)dim * (1 << bits);
-    return launch_merge(p, msmem, 0, st);
+    return launch_merge(p, false, msmem, 0, st);
 }
 
 extern "C" size_t tqb_scan_topk_prod_workspace_bytes(int nq, int64_t n, int dim, int bits, int k) {
     if (nq <= 0 || dim <= 0 || bits < 2 || bits > 5 || k <= 0 || k > TQB_SCAN_MAX_K) return 0;
     // the MSE scan's workspace plus the queries projected by the QJL matrix
     return tqb::plan_scan(nq, n, dim, bits - 1, k).total + tqb::s_align((size_t)nq * dim * 4) +
-           tqb::scan_tc_plan(nq, dim, true, k, k + tqb::SCAN_SELECT_MARGIN).total;
+           tqb::scan_tc_plan(nq, dim, true, k + tqb::SCAN_SELECT_MARGIN).total;
 }
 
 extern "C" int tqb_scan_topk_prod(const float* queries, int nq, const uint8_t* mse_packed, const uint8_t* signs,
@@ -1407,7 +1459,7 @@ extern "C" int tqb_scan_topk_prod(const float* queries, int nq, const uint8_t* m
     const int mb = bits - 1;
     const ScanPlan pl = plan_scan(nq, n, dim, mb, k);
     const int ksel = k + SCAN_SELECT_MARGIN;
-    const ScanTcPlan tpl = scan_tc_plan(nq, dim, true, k, ksel);
+    const ScanTcPlan tpl = scan_tc_plan(nq, dim, true, ksel);
     const size_t tc_off = pl.total + s_align((size_t)nq * dim * 4), need = tc_off + tpl.total;
     if (workspace_bytes < need)
         return fail(TQB_ERR_WORKSPACE, "scan_topk_prod: workspace %zu bytes < required %zu", workspace_bytes, need);
@@ -1442,22 +1494,22 @@ extern "C" int tqb_scan_topk_prod(const float* queries, int nq, const uint8_t* m
     if (int e = check_launch("scan_prepare")) return e;
 
     // (rows of whole 4-byte words, as the tensor-core pass reads them)
-    if (((uintptr_t)mse_packed | (uintptr_t)signs) % 4 == 0 && scan_tc_wanted(nq, n - n % SCAN_TILE, dim, mb, true, ksel)) {
+    const size_t msmem = sizeof(float) * (size_t)dim * (1 << mb);
+    if (((uintptr_t)mse_packed | (uintptr_t)signs) % 4 == 0 && scan_tc_wanted(nq, n - n % SCAN_TILE, dim, mb, true, ksel, true)) {
         ScanTcArgs t{};
         t.packed = mse_packed; t.norms = norms; t.signs = signs; t.res_norms = res_norms; t.sign_coef = p.sign_coef;
-        t.rows = n - n % SCAN_TILE; t.dim = dim; t.bits = mb; t.nq = nq; t.k = k; t.ksel = ksel; t.cent = centroids;
-        t.qrot = p.qrot; t.qsign = qsign;
+        t.rows = n - n % SCAN_TILE; t.dim = dim; t.bits = mb; t.nq = nq; t.ksel = ksel; t.cent = centroids;
+        t.qrot = p.qrot; t.qsign = qsign; t.proven = true;
         if (int e = scan_tc_run(t, tpl, ws + tc_off, st)) return e;
-        p.buf_n = reinterpret_cast<const int*>(ws + tc_off + tpl.off_count); p.buf_cap = tpl.cap;
-        p.buf_s = reinterpret_cast<const float*>(ws + tc_off + tpl.off_s); p.buf_i = reinterpret_cast<const int*>(ws + tc_off + tpl.off_i);
+        take_buffers(p, tpl, ws + tc_off, true);
+        if (int e = launch_merge(p, true, msmem, 0, st)) return e;
     }
     const size_t smem = sizeof(float) * ((size_t)dim * (1 << mb) + dim) + (size_t)SCAN_WARPS * p.kk * 8;
     TQB_CUDA(cudaFuncSetAttribute(scan_generic_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     dim3 grid(gx, nq);
     scan_generic_kernel<<<grid, SCAN_WARPS * 32, smem, st>>>(p);
     if (int e = check_launch("scan_generic")) return e;
-    const size_t msmem = sizeof(float) * (size_t)dim * (1 << mb);
-    return launch_merge(p, msmem, 0, st);
+    return launch_merge(p, false, msmem, 0, st);
 }
 
 extern "C" int tqb_topk_merge(const float* scores, const int64_t* ids, int nq, int parts, int k,

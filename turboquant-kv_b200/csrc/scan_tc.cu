@@ -6,6 +6,12 @@
 // queries (Prod: 128) lie in shared memory as the B operand.  The pass ranks only, like the passes of scan.cu: the merge
 // re-scores the best k + 24 candidates in float32, and the scores it reports come from there.
 //
+// The list kernels rank Prod rows in float32, and MSE rows with queries of 22 bits where k > 24; here every operand has 11.
+// Those calls' selections are PROVEN: with E a bound of |approximate - float32 score| (scan_tc_error), no row below the k-th
+// best approximate score by more than 2 E can be among the best k, so everything above that is re-scored; where the buffer
+// does not reach that far down (rows closer together than fp16 tells apart), the list kernels answer the query.  MSE calls of
+// k <= 24 rank as they do there, on fp16 centroids and queries with the margin of 24.
+//
 // Candidates without lists: keeping sorted lists costs about k ln(rows) insertions per query and list, which bounds the other
 // passes.  Here a first launch scores every `stride`-th tile and keeps only the largest score of each group of rows; the
 // ksel-th largest of those maxima is not above the ksel-th best score of all rows (the maxima belong to distinct rows), and
@@ -76,8 +82,9 @@ __device__ __forceinline__ uint32_t st_field(const uint32_t (&w)[NW], int bit, i
 // One block per column (padded columns are zero).  The scale is the query's own: scores of one query are only compared
 // with one another.
 __global__ void __launch_bounds__(128) scan_tc_image_kernel(const ScanTcArgs a) {
-    __shared__ float red[4];
+    __shared__ float red[4], sums[2][4];
     const int col = blockIdx.x, q = col, d = threadIdx.x;
+    if (col == 0 && d < 2) a.limits[d] = 0;
     const bool prod = a.signs != nullptr, live = q < a.nq && d < a.dim;
     const float x = live ? a.qrot[(int64_t)q * a.dim + d] : 0.0f, y = live && prod ? a.qsign[(int64_t)q * a.dim + d] : 0.0f;
     float mx = fmaxf(fabsf(x), fabsf(y));
@@ -93,10 +100,17 @@ __global__ void __launch_bounds__(128) scan_tc_image_kernel(const ScanTcArgs a) 
         *reinterpret_cast<__half*>(img + off) = __float2half_rn(x * sc);
         if (prod) *reinterpret_cast<__half*>(img + kblk * a.cols * 128 + off) = __float2half_rn(y * sc);
     }
+    float sx = fabsf(x * sc), sy = fabsf(y * sc);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) { sx += __shfl_xor_sync(0xffffffffu, sx, o); sy += __shfl_xor_sync(0xffffffffu, sy, o); }
+    if ((d & 31) == 0) { sums[0][d >> 5] = sx; sums[1][d >> 5] = sy; }
+    __syncthreads();
+    if (d == 0 && q < a.nq)
+        a.qsum[q] = make_float2((sums[0][0] + sums[0][1]) + (sums[0][2] + sums[0][3]), (sums[1][0] + sums[1][1]) + (sums[1][2] + sums[1][3]));
 }
 
 // ---- bound of every query from the sample's group maxima --------------------------------------------
-// First the ksel-th largest of the threads' own maxima, a lower bound that leaves few values; then the exact rank among those.
+// First the rank-th largest of the threads' own maxima, a lower bound that leaves few values; then the exact rank among those.
 __global__ void __launch_bounds__(256) scan_tc_threshold_kernel(const ScanTcArgs a) {
     extern __shared__ float g[];
     __shared__ float top[256], bound, low;
@@ -110,7 +124,7 @@ __global__ void __launch_bounds__(256) scan_tc_threshold_kernel(const ScanTcArgs
     int rank = 0;
 #pragma unroll 8
     for (int o = 0; o < 256; o++) rank += (top[o] > v || (top[o] == v && o < t)) ? 1 : 0;
-    if (rank == a.ksel - 1) low = v;                       // (never with more than 256 wanted: then all values are ranked)
+    if (rank == a.rank - 1) low = v;                       // (never with more than 256 wanted: then all values are ranked)
     __syncthreads();
     for (int i = t; i < a.groups; i += 256) {
         const float x = a.gmax[(int64_t)q * a.groups + i];
@@ -122,7 +136,7 @@ __global__ void __launch_bounds__(256) scan_tc_threshold_kernel(const ScanTcArgs
         const float x = g[i];
         int r = 0;
         for (int o = 0; o < n; o++) r += (g[o] > x || (g[o] == x && o < i)) ? 1 : 0;
-        if (r == a.ksel - 1) bound = x;                    // (ranks are distinct)
+        if (r == a.rank - 1) bound = x;                    // (ranks are distinct)
     }
     __syncthreads();
     if (t == 0) {
@@ -215,7 +229,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) scan_tc_kernel(const ScanTcArgs
         constexpr int HW = D / 64;                         // plane words of half a row
         const int half = lane >> 4, trow = warp * 16 + (lane & 15), bpp = D / 8;
         uint32_t w[PROD ? 1 : NW], wn[PROD ? 1 : NW], pw[HW][4], pn[HW][4], sg[HW], sn[HW];
-        float res = 0.0f, resn = 0.0f;
+        float res = 0.0f, resn = 0.0f, top_sign = 0.0f;    // (top_sign: largest magnitude of the sign operand)
         auto request = [&](int64_t tile) {
             if constexpr (PROD) {
                 const int64_t r = tile * ST_TILE + trow;
@@ -260,7 +274,9 @@ __global__ void __launch_bounds__(ST_THREADS, 1) scan_tc_kernel(const ScanTcArgs
             if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
             const uint32_t at = base + C::OFF_A + b * C::A_BUF;
             if constexpr (PROD) {
-                const uint32_t h = __half_as_ushort(__float2half_rn(fminf(a.sign_coef * res * csc, 60000.0f))), neg = (h | (h << 16)) ^ 0x80008000u;
+                const float mag = a.sign_coef * res * csc;
+                if (!SAMPLE) top_sign = fmaxf(top_sign, fabsf(mag) > 60000.0f ? -ST_NEG_INF : fabsf(mag));  // (beyond fp16: no bound; NaN: no score)
+                const uint32_t h = __half_as_ushort(__float2half_rn(mag > 60000.0f ? 60000.0f : mag)), neg = (h | (h << 16)) ^ 0x80008000u;
 #pragma unroll
                 for (int i = 0; i < HW; i++) {
                     uint32_t X[4];
@@ -292,6 +308,10 @@ __global__ void __launch_bounds__(ST_THREADS, 1) scan_tc_kernel(const ScanTcArgs
             __syncwarp();
             if (lane == 0) st_arrive(a_ready(b));
         }
+        if (PROD && !SAMPLE && blockIdx.y == 0) {
+            top_sign = st_warp_max(top_sign);
+            if (lane == 0) atomicMax(a.limits + 1, __float_as_uint(top_sign));
+        }
     } else if (warp < ST_DEC + ST_EPI) {
         // ================= epilogue: thread = row, half of the columns =================
         const int ew = warp & 3, half = (warp - ST_DEC) >> 2, row = ew * 32 + lane;
@@ -299,6 +319,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) scan_tc_kernel(const ScanTcArgs
         const uint32_t thr_at = base + C::OFF_THR + col0 * 4;
         uint32_t it = 0;
         float mine[4] = {ST_NEG_INF, ST_NEG_INF, ST_NEG_INF, ST_NEG_INF};       // SAMPLE: group maxima of columns 32 i + lane
+        float top_norm = 0.0f;                             // largest |norm| of the thread's rows
         int flush = 0;
         auto put_group = [&]() {
 #pragma unroll
@@ -334,6 +355,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) scan_tc_kernel(const ScanTcArgs
             if (r < a.rows)
                 nrm = PROD ? __ldg(a.norms + r)
                            : __ldg(reinterpret_cast<const float*>(a.records + (r >> 4) * a.rec_bytes + tl_key_section(D, BITS ? BITS : 4) + tl_norm_offset(0, 0, (int)(r & 15))));
+            if (!SAMPLE) top_norm = fmaxf(top_norm, fabsf(nrm));           // (NaN: passed over)
             ok = mbar_wait(acc_full(b), (it >> 1) & 1);
             if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
             tc_fence_after();
@@ -402,10 +424,15 @@ __global__ void __launch_bounds__(ST_THREADS, 1) scan_tc_kernel(const ScanTcArgs
             if (lane == 0) st_arrive(acc_free(b));
             if (SAMPLE && (it + 1) % a.tiles_per_flush == 0) put_group();
         }
-        if (SAMPLE)
+        if (SAMPLE) {
             while (flush < a.flushes) put_group();         // (what is left, then groups without rows)
-        else
+        } else {
             take_places();
+            if (blockIdx.y == 0 && half == 0) {
+                top_norm = st_warp_max(top_norm);
+                if (lane == 0) atomicMax(a.limits, __float_as_uint(top_norm));
+            }
+        }
     } else if (lane == 0) {
         // ================= MMA issuer (one lane) =================
         const uint32_t bbytes = (uint32_t)(KBLK * a.cols * 128);
@@ -445,7 +472,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) scan_tc_kernel(const ScanTcArgs
 
 static size_t st_align(size_t v) { return (v + 255) / 256 * 256; }
 
-ScanTcPlan scan_tc_plan(int nq, int dim, bool prod, int k, int ksel) {
+ScanTcPlan scan_tc_plan(int nq, int dim, bool prod, int ksel) {
     ScanTcPlan pl{};
     const int most = prod ? ST_MAX_COLS_PROD : ST_MAX_COLS;
     pl.blocks = (int)ceil_div(nq, most);
@@ -460,10 +487,11 @@ ScanTcPlan scan_tc_plan(int nq, int dim, bool prod, int k, int ksel) {
     pl.off_gmax = off;   off = st_align(off + (size_t)nq * ST_GROUPS_MAX * 4);
     pl.off_thr = off;    off = st_align(off + (size_t)nq * 4);
     pl.off_count = off;  off = st_align(off + (size_t)nq * 4);
+    pl.off_limits = off; off = st_align(off + 2 * 4);
+    pl.off_qsum = off;   off = st_align(off + (size_t)nq * sizeof(float2));
     pl.off_s = off;      off = st_align(off + (size_t)nq * pl.cap * 4);
     pl.off_i = off;      off = st_align(off + (size_t)nq * pl.cap * 4);
     pl.total = off;
-    (void)k;
     return pl;
 }
 
@@ -471,11 +499,13 @@ ScanTcPlan scan_tc_plan(int nq, int dim, bool prod, int k, int ksel) {
 // are sampled whole.
 static int st_stride(int64_t rows, int ksel) { return (int)std::max<int64_t>(1, std::min<int64_t>(ST_MAX_STRIDE, rows / ST_TILE / ksel)); }
 
-bool scan_tc_wanted(int nq, int64_t rows, int dim, int bits, bool prod, int ksel) {
+bool scan_tc_wanted(int nq, int64_t rows, int dim, int bits, bool prod, int ksel, bool proven) {
     if ((dim != 64 && dim != 128) || bits < (prod ? 1 : 2) || bits > 4) return false;
     // Two groups of rows per wanted candidate at least.  From nine queries (two passes of the list kernels) on: 8 queries over
     // 1 M x d128 rows 207 us there, 16 here 124 us; 5,000 rows, 30 queries 141 us there.  Prod rows: the list kernel scores a row a lane.
     if (4 * (rows / ST_TILE) < 2 * ksel) return false;
+    // (a proof wants room below the k-th best score: twice the groups where k is large against the margin)
+    if (proven && ksel > 64 && 4 * (rows / ST_TILE) < 4 * ksel) return false;
     return prod || nq >= 9;
 }
 
@@ -500,6 +530,7 @@ int scan_tc_run(ScanTcArgs a, const ScanTcPlan& pl, uint8_t* ws, cudaStream_t st
     a.images = ws + pl.off_images; a.gmax = reinterpret_cast<float*>(ws + pl.off_gmax); a.thr = reinterpret_cast<float*>(ws + pl.off_thr);
     a.count = reinterpret_cast<int*>(ws + pl.off_count); a.buf_s = reinterpret_cast<float*>(ws + pl.off_s);
     a.buf_i = reinterpret_cast<int*>(ws + pl.off_i);
+    a.limits = reinterpret_cast<uint32_t*>(ws + pl.off_limits); a.qsum = reinterpret_cast<float2*>(ws + pl.off_qsum);
     a.cap = pl.cap; a.cols = pl.cols; a.blocks = pl.blocks;
     a.stride = st_stride(a.rows, a.ksel);
     const int64_t sampled = ceil_div(ceil_div(a.rows, ST_TILE), a.stride);
@@ -511,6 +542,9 @@ int scan_tc_run(ScanTcArgs a, const ScanTcPlan& pl, uint8_t* ws, cudaStream_t st
     a.tiles_per_flush = (int)ceil_div(per_cta, want);
     a.flushes = (int)ceil_div(per_cta, a.tiles_per_flush);
     a.groups = 4 * a.gx * a.flushes;
+    // The bound's rank among the sample's maxima: small indexes, sampled densely, take it lower (the buffer expects the
+    // candidates of a stride of 16), so that a selection finds room below the k-th best score.
+    a.rank = a.proven ? std::max(a.ksel, std::min(a.groups / 2, a.ksel * std::max(1, 4 / a.stride))) : a.ksel;
     if (int e = tc_error_word(&a.error)) return e;
     scan_tc_image_kernel<<<a.cols * a.blocks, 128, 0, st>>>(a);
     if (int e = check_launch("scan_tc_image")) return e;
