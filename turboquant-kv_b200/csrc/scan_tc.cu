@@ -84,7 +84,7 @@ __device__ __forceinline__ uint32_t st_field(const uint32_t (&w)[NW], int bit, i
 __global__ void __launch_bounds__(128) scan_tc_image_kernel(const ScanTcArgs a) {
     __shared__ float red[4], sums[2][4];
     const int col = blockIdx.x, q = col, d = threadIdx.x;
-    if (col == 0 && d < 2) a.limits[d] = 0;
+    if (col == 0 && d < 3) a.limits[d] = 0;
     const bool prod = a.signs != nullptr, live = q < a.nq && d < a.dim;
     const float x = live ? a.qrot[(int64_t)q * a.dim + d] : 0.0f, y = live && prod ? a.qsign[(int64_t)q * a.dim + d] : 0.0f;
     float mx = fmaxf(fabsf(x), fabsf(y));
@@ -143,8 +143,8 @@ __global__ void __launch_bounds__(256) scan_tc_threshold_kernel(const ScanTcArgs
         // the main launch compares unrounded products with it: a little lower, so that the bound's own row stays (and finite,
         // so that infinite scores are not below it)
         a.thr[q] = fminf(bound, 3.4e38f) - fabsf(fminf(bound, 3.4e38f)) * 2e-6f;
-        // the list kernels answer where the sample gave no bound (rows or queries that are not numbers)
-        a.count[q] = bound == ST_NEG_INF ? a.cap + 1 : 0;
+        // the list kernels answer where the sample gave up or gave no bound (rows or queries that are not numbers)
+        a.count[q] = a.limits[2] || bound == ST_NEG_INF ? a.cap + 1 : 0;
     }
 }
 
@@ -460,7 +460,12 @@ __global__ void __launch_bounds__(ST_THREADS, 1) scan_tc_kernel(const ScanTcArgs
         // (an unfinished copy must not outlive the block: the wait above is bounded, and so is this one)
         if (!ok) mbar_wait(b_full, 0);
     }
-    if (!ok && lane == 0) atomicExch(a.error, 1);
+    if (!ok && lane == 0) {
+        atomicExch(a.error, 1);
+        if (SAMPLE) atomicExch(a.limits + 2, 1u);
+        else
+            for (int q = q0; q < min(a.nq, q0 + a.cols); q++) atomicMax(a.count + q, a.cap + 1);      // the list kernels answer
+    }
     __syncwarp();
     tc_fence_before();
     __syncthreads();
@@ -487,7 +492,7 @@ ScanTcPlan scan_tc_plan(int nq, int dim, bool prod, int ksel) {
     pl.off_gmax = off;   off = st_align(off + (size_t)nq * ST_GROUPS_MAX * 4);
     pl.off_thr = off;    off = st_align(off + (size_t)nq * 4);
     pl.off_count = off;  off = st_align(off + (size_t)nq * 4);
-    pl.off_limits = off; off = st_align(off + 2 * 4);
+    pl.off_limits = off; off = st_align(off + 3 * 4);
     pl.off_qsum = off;   off = st_align(off + (size_t)nq * sizeof(float2));
     pl.off_s = off;      off = st_align(off + (size_t)nq * pl.cap * 4);
     pl.off_i = off;      off = st_align(off + (size_t)nq * pl.cap * 4);

@@ -14,7 +14,7 @@ struct ScanTcArgs {
     // workspace
     uint8_t* images; float* gmax; float* thr;
     int* count; float* buf_s; int* buf_i; int cap;         // candidates of a query: count[q], then buf_*[q * cap ..]
-    uint32_t* limits;                                      // largest |norm| and sign magnitude of the rows (float bits)
+    uint32_t* limits;                                      // largest |norm| and sign magnitude of the rows (float bits), 1 = a wait expired
     float2* qsum;                                          // sums of the magnitudes of a query's two (scaled) columns
     int* error;
     // plan (gx: CTAs of a query block in the sampling launch)
@@ -27,7 +27,8 @@ ScanTcPlan scan_tc_plan(int nq, int dim, bool prod, int ksel);
 // Whether the pass is taken for this call (the reasons are in scan_tc.cu).  `proven`: its selection has to be proven, see below.
 bool scan_tc_wanted(int nq, int64_t rows, int dim, int bits, bool prod, int ksel, bool proven);
 // Candidates of every query into its buffer: everything not below a bound (thr) of the ksel-th best approximate score.  A query
-// with count[q] > cap has overflowed (more rows tie with the bound than the buffer holds): its buffer is not used.
+// with count[q] > cap has overflowed (more rows tie with the bound than the buffer holds, or a wait expired): its buffer is
+// not used.
 int scan_tc_run(ScanTcArgs a, const ScanTcPlan& pl, uint8_t* ws, cudaStream_t st);
 
 // Largest difference between a row's approximate score (in its query's scale) and its float32 score, for rows whose norms and
