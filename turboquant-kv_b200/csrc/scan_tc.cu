@@ -37,7 +37,6 @@ constexpr int ST_MAX_COLS = 256, ST_MAX_COLS_PROD = 128;
 constexpr int ST_MAX_STRIDE = 16;
 constexpr int ST_LOG = 96;                     // candidates an epilogue warp gathers before it takes places in the buffers
 constexpr int ST_GROUPS = 512;                // group maxima per query, at least (four per wanted candidate where k is large)
-constexpr int ST_GROUPS_MAX = 4096;
 constexpr float ST_NEG_INF = -__builtin_huge_valf();
 
 template <int D, bool PROD>
@@ -477,8 +476,12 @@ __global__ void __launch_bounds__(ST_THREADS, 1) scan_tc_kernel(const ScanTcArgs
 
 static size_t st_align(size_t v) { return (v + 255) / 256 * 256; }
 
+// Group maxima of a query at most, as scan_tc_run deals them.
+static int st_groups(int ksel, int gx) { return std::max(ST_GROUPS, 4 * ksel) + 4 * gx; }
+
 ScanTcPlan scan_tc_plan(int nq, int dim, bool prod, int ksel) {
     ScanTcPlan pl{};
+    if (!prod && nq < SCAN_TC_MIN_QUERIES) return pl;
     const int most = prod ? ST_MAX_COLS_PROD : ST_MAX_COLS;
     pl.blocks = (int)ceil_div(nq, most);
     pl.cols = (int)ceil_div(ceil_div(nq, pl.blocks), 32) * 32;
@@ -489,7 +492,7 @@ ScanTcPlan scan_tc_plan(int nq, int dim, bool prod, int ksel) {
     while (pl.cap < 6 * ksel * ST_MAX_STRIDE) pl.cap *= 2;
     size_t off = 0;
     pl.off_images = off; off = st_align(off + (size_t)pl.blocks * pl.cols * dim * 2 * (prod ? 2 : 1));
-    pl.off_gmax = off;   off = st_align(off + (size_t)nq * ST_GROUPS_MAX * 4);
+    pl.off_gmax = off;   off = st_align(off + (size_t)nq * st_groups(ksel, pl.gx) * 4);
     pl.off_thr = off;    off = st_align(off + (size_t)nq * 4);
     pl.off_count = off;  off = st_align(off + (size_t)nq * 4);
     pl.off_limits = off; off = st_align(off + 3 * 4);
@@ -511,7 +514,7 @@ bool scan_tc_wanted(int nq, int64_t rows, int dim, int bits, bool prod, int ksel
     if (4 * (rows / ST_TILE) < 2 * ksel) return false;
     // (a proof wants room below the k-th best score: twice the groups where k is large against the margin)
     if (proven && ksel > 64 && 4 * (rows / ST_TILE) < 4 * ksel) return false;
-    return prod || nq >= 9;
+    return prod || nq >= SCAN_TC_MIN_QUERIES;
 }
 
 template <int D, int BITS, bool PROD>
@@ -543,7 +546,7 @@ int scan_tc_run(ScanTcArgs a, const ScanTcPlan& pl, uint8_t* ws, cudaStream_t st
     const int64_t per_cta = ceil_div(sampled, a.gx);       // sampled tiles of a CTA
     // four groups per CTA and flush: enough of them, no more than the buffer holds
     int64_t want = ceil_div(std::max(ST_GROUPS, 4 * a.ksel), 4 * a.gx);
-    want = std::min<int64_t>(std::min<int64_t>(want, per_cta), std::max(1, ST_GROUPS_MAX / (4 * a.gx)));
+    want = std::min<int64_t>(want, per_cta);
     a.tiles_per_flush = (int)ceil_div(per_cta, want);
     a.flushes = (int)ceil_div(per_cta, a.tiles_per_flush);
     a.groups = 4 * a.gx * a.flushes;

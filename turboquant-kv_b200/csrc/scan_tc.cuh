@@ -22,7 +22,8 @@ struct ScanTcArgs {
 };
 struct ScanTcPlan { size_t off_images, off_gmax, off_thr, off_count, off_limits, off_qsum, off_s, off_i, total; int cap, cols, blocks, gx; };
 
-// Workspace and shape of the pass; independent of the number of rows.
+constexpr int SCAN_TC_MIN_QUERIES = 9;                     // MSE calls of fewer queries never take the pass
+// Workspace and shape of the pass (nothing for such calls); independent of the number of rows.
 ScanTcPlan scan_tc_plan(int nq, int dim, bool prod, int ksel);
 // Whether the pass is taken for this call (the reasons are in scan_tc.cu).  `proven`: its selection has to be proven, see below.
 bool scan_tc_wanted(int nq, int64_t rows, int dim, int bits, bool prod, int ksel, bool proven);
