@@ -46,3 +46,36 @@ def test_same_rows_as_the_ffma_kernel(orc, dim, bits, rows, dtype):
         for t in range(8):
             if (bits_off >> (7 - t)) & 1:
                 assert abs(proj[8 * j + t]) < 4e-6 * np.linalg.norm(S[8 * j + t].double().cpu().numpy())
+
+
+def _both(x, bits, rot, S):
+    """(tensor-core call, FFMA calls of a few hundred rows) of the same rows."""
+    from turboquant_kv import reference as R
+
+    dim = x.shape[1]
+    how = {"rotation": rot, "codebook": tuple(t.cuda() for t in R.lloyd_max_codebook(bits - 1, dim)), "S_matrix": S}
+    small = [R.quantize_prod(x[i:i + SMALL], bits, **how) for i in range(0, x.shape[0], SMALL)]
+    return R.quantize_prod(x, bits, **how), tuple(torch.cat([t[k] for t in small]) for k in range(4))
+
+
+@pytest.mark.parametrize("dim,bits", [(128, 2), (128, 4), (64, 3), (96, 2)])
+def test_codes_where_the_two_sums_differ_most(dim, bits):
+    """Rows whose coordinate 5 is a difference of large partial sums, within a few roundings of the middle boundary; and a
+    rotation with rows of very different lengths, whose coordinates differ by more than a unit vector's."""
+    from turboquant_kv import reference as R
+
+    gen = torch.Generator(device="cuda").manual_seed(dim + bits)
+    rot = R.make_rotation_matrix(dim, 42).cuda()
+    S = R._make_qjl_matrix(dim, dim, 42, torch.device("cuda"))
+    r = rot[5].double()
+    flip = torch.ones(dim, device="cuda", dtype=torch.float64)
+    flip[dim // 2:] = -1.0
+    x = (r * flip)[None, :] + 0.05 * torch.randn(40_000, dim, generator=gen, device="cuda", dtype=torch.float64)
+    x -= (x @ r)[:, None] * r                                   # coordinate 5 is zero ...
+    x += 2e-7 * torch.randn(40_000, 1, generator=gen, device="cuda", dtype=torch.float64) * r      # ... but for this
+    got, want = _both(x.float(), bits, rot, S)
+    assert torch.equal(got[0], want[0]) and torch.equal(got[3], want[3])
+    scale = torch.exp(torch.linspace(-6.0, 6.0, dim, device="cuda"))[:, None]
+    y = torch.randn(60_000, dim, generator=gen, device="cuda")
+    got, want = _both(y, bits, (rot * scale).contiguous(), S)
+    assert torch.equal(got[0], want[0]) and torch.equal(got[3], want[3])

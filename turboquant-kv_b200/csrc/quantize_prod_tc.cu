@@ -5,8 +5,8 @@
 //
 // Codes are those of the float32 chain of quantize.cu: u is its unit vector to the bit; both operands of the rotation enter
 // as two fp16 terms (22 bits, scaled by powers of two), three products summed in float32, low orders first; a coordinate
-// closer to a decision boundary than QP_ABS + QP_REL |y| -- ten times what was seen between the two -- is computed again by
-// that chain (about one in a hundred thousand).  A sign may fall the other way where the projection is zero to within
+// closer to a decision boundary than the two can differ by (QP_CHAIN, QP_TERMS below) is computed again by that chain: one in
+// 5,000 at two bits, in 1,100 at four.  A sign may fall the other way where the projection is zero to within
 // float32 rounding, about 1e-7 of ||e||, as it may between any two float32 orders.
 //
 // What bounds it (d = 128, float32, 2 bits + sign; clocks of a 128-row tile on one SM): 2 x 1,536 on the tensor cores, 2,600
@@ -22,7 +22,13 @@ namespace tqb {
 
 constexpr int QP_TILE = 128, QP_WARPS = 16, QP_THREADS = QP_WARPS * 32, QP_RPW = QP_TILE / QP_WARPS;
 constexpr int QP_LIST = 1024;                 // coordinates computed again in one go
-constexpr float QP_ABS = 3e-7f, QP_REL = 2e-6f;
+// Bound of the difference between a coordinate and the float32 chain's, in units of ||row of R|| (sum |u_k R_jk| is at most
+// that, ||u|| being one to within rounding; 2 % more covers it).  The chain: dim roundings of 2^-24.  The terms: either
+// operand is off by 2^-22 of itself, the product of the low terms, 2^-22, is left out, and the accumulators round toward zero,
+// up to 2^-22 after each of the dim / 16 MMAs of the leading product (the others are 2^-11 of it) and once more for their sum.
+// Beside it sqrt(dim) 2^-25 of either operand's scale, for terms below fp16's normal range.
+constexpr float QP_UNIT = 1.02f / 4194304.0f;                                    // 2^-22
+__host__ __device__ constexpr float qp_guard(int dim) { return QP_UNIT * (0.25f * dim + 3.0f + dim / 16.0f + 1.0f); }
 
 struct ProdArgs {
     const void* x; int64_t n, x_stride;
@@ -40,7 +46,8 @@ struct QpCfg {
     static constexpr int OFF_LIST = OFF_SIGNS + QP_TILE * W * 4;
     static constexpr int OFF_ROW = OFF_LIST + QP_LIST * 4;                       // den, ||u||, 4 partial sums of e^2
     static constexpr int OFF_CB = OFF_ROW + 6 * QP_TILE * 4;                     // boundaries, centroids
-    static constexpr int OFF_BAR = OFF_CB + 128;
+    static constexpr int OFF_GUARD = OFF_CB + 128;                               // guard of every coordinate
+    static constexpr int OFF_BAR = OFF_GUARD + DP * 4;
     static constexpr int TOTAL = OFF_BAR + 64 + 1024;                            // + slack for the 1024-byte alignment
     static constexpr int CG = DP / 4;                                            // columns of an epilogue thread
     static_assert(TOTAL <= 227 * 1024, "shared memory");
@@ -56,13 +63,26 @@ __device__ __forceinline__ void qp_split2(float a, float b, uint32_t& hi, uint32
     lo = pack_half2(a - f.x, b - f.y);
 }
 // K-major, 128-byte-swizzled B operand of M (row n = output, column k = contraction), hi and lo terms; returns the scale.
+// len (or null): the rows' lengths.
 template <int DP>
-__device__ __forceinline__ float qp_build(uint8_t* sm, int off_hi, int off_lo, const float* __restrict__ M, int dim, float* red) {
+__device__ __forceinline__ float qp_build(uint8_t* sm, int off_hi, int off_lo, const float* __restrict__ M, int dim, float* red, float* len) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float mx = 0.0f;
-    for (int i = threadIdx.x; i < dim * dim; i += QP_THREADS) mx = fmaxf(mx, fabsf(__ldg(M + i)));
+    for (int n = warp; n < dim; n += QP_WARPS) {
+        float ss = 0.0f;
+        for (int k = lane; k < dim; k += 32) {
+            const float v = __ldg(M + (int64_t)n * dim + k);
+            mx = fmaxf(mx, fabsf(v));
+            ss = fmaf(v, v, ss);
+        }
+        if (len) {
+            ss = sqrtf(warp_sum(ss));
+            if (lane == 0) len[n] = ss;
+        }
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
+    if (lane == 0) red[warp] = mx;
     __syncthreads();
     mx = 0.0f;
     for (int w = 0; w < QP_WARPS; w++) mx = fmaxf(mx, red[w]);
@@ -102,8 +122,13 @@ __global__ void __launch_bounds__(QP_THREADS, 1) quantize_prod_tc_kernel(const P
     float* const cent_s = bnd_s + 16;
     if (threadIdx.x < NB) bnd_s[threadIdx.x] = a.bnd[threadIdx.x];
     if (threadIdx.x <= NB) cent_s[threadIdx.x] = a.cent[threadIdx.x];
-    const float unscale = 1.0f / (USC * qp_build<DP>(sm, C::OFF_R, C::OFF_R + C::TERM, a.rot, a.dim, red));
-    qp_build<DP>(sm, C::OFF_T, C::OFF_T + C::TERM, a.qjl_rot, a.dim, red);       // (its product is used for its sign only)
+    float* const guard_s = reinterpret_cast<float*>(sm + C::OFF_GUARD);
+    if (threadIdx.x < DP) guard_s[threadIdx.x] = -1.0f;    // (columns beyond dim: never)
+    __syncthreads();
+    const float rsc = qp_build<DP>(sm, C::OFF_R, C::OFF_R + C::TERM, a.rot, a.dim, red, guard_s);
+    const float unscale = 1.0f / (USC * rsc);
+    if (threadIdx.x < a.dim) guard_s[threadIdx.x] = fmaf(qp_guard(a.dim), guard_s[threadIdx.x], 12.0f * 2.9802322e-8f * (1.0f / rsc + guard_s[threadIdx.x] / USC));
+    qp_build<DP>(sm, C::OFF_T, C::OFF_T + C::TERM, a.qjl_rot, a.dim, red, nullptr);      // (its product is used for its sign only)
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     tc_fence_before();
     __syncthreads();
@@ -266,6 +291,8 @@ __global__ void __launch_bounds__(QP_THREADS, 1) quantize_prod_tc_kernel(const P
             for (int c = 0; c < CG; c += 8) {
                 uint32_t v[8], v2[8], h[4], l[4];
                 float e[8];
+                const float4 ga = *reinterpret_cast<const float4*>(guard_s + col0 + c), gb = *reinterpret_cast<const float4*>(guard_s + col0 + c + 4);
+                const float gd[8] = {ga.x, ga.y, ga.z, ga.w, gb.x, gb.y, gb.z, gb.w};
                 tmem_ld8_async(src + c, v);
                 tmem_ld8(src + DP + c, v2);                // (waits for both)
                 tmem_wait8(v);
@@ -282,7 +309,7 @@ __global__ void __launch_bounds__(QP_THREADS, 1) quantize_prod_tc_kernel(const P
                         near = fminf(near, fabsf(y - bnd[b]));
                     }
                     const bool in = col0 + c + i < a.dim;
-                    if (in && near < fmaf(QP_REL, fabsf(y), QP_ABS)) guard |= 1u << (c + i);
+                    if (near < gd[i]) guard |= 1u << (c + i);
                     e[i] = in ? fmaf(n2, y, -cv) : 0.0f;
                     ee = fmaf(e[i], e[i], ee);
                     const int bit = 8 * (c >> 3) + 7 - i;
