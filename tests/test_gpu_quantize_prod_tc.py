@@ -79,3 +79,17 @@ def test_codes_where_the_two_sums_differ_most(dim, bits):
     y = torch.randn(60_000, dim, generator=gen, device="cuda")
     got, want = _both(y, bits, (rot * scale).contiguous(), S)
     assert torch.equal(got[0], want[0]) and torch.equal(got[3], want[3])
+
+
+@pytest.mark.parametrize("dim,bits,dtype", [(128, 3, "f32"), (64, 2, "bf16"), (96, 4, "f16")])
+def test_blocks_of_zero_and_non_finite_rows(dim, bits, dtype):
+    """Whole tiles of zero rows (a padded database), infinities and NaN: the bytes of the FFMA kernel."""
+    from turboquant_kv import reference as R
+
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.randn(3000, dim, generator=gen, device="cuda")
+    x[200:1700] = 0.0
+    x[1800, 3], x[1801, 4], x[1802, 5] = float("inf"), float("-inf"), float("nan")
+    got, want = _both(x.to(DTYPES[dtype]), bits, R.make_rotation_matrix(dim, 42).cuda(), R._make_qjl_matrix(dim, dim, 42, torch.device("cuda")))
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1][200:1700], want[1][200:1700]) and torch.equal(got[1][1800:1803], want[1][1800:1803])
+    assert torch.equal(got[3].nan_to_num(-1.0), want[3].nan_to_num(-1.0)) and torch.equal(got[2].isnan(), want[2].isnan())

@@ -6,7 +6,7 @@
 // Codes are those of the float32 chain of quantize.cu: u is its unit vector to the bit; both operands of the rotation enter
 // as two fp16 terms (22 bits, scaled by powers of two), three products summed in float32, low orders first; a coordinate
 // closer to a decision boundary than the two can differ by (QP_CHAIN, QP_TERMS below) is computed again by that chain: one in
-// 5,000 at two bits, in 1,100 at four.  A sign may fall the other way where the projection is zero to within
+// 5,000 at two bits, in 1,100 at four.  (A zero row is zero on both sides: not again.)  A sign may fall the other way where the projection is zero to within
 // float32 rounding, about 1e-7 of ||e||, as it may between any two float32 orders.
 //
 // What bounds it (d = 128, float32, 2 bits + sign; clocks of a 128-row tile on one SM): 2 x 1,536 on the tensor cores, 2,600
@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(QP_THREADS, 1) quantize_prod_tc_kernel(const P
                 else reinterpret_cast<uint16_t*>(planes)[(row * MB + p) * (2 * words) + cg] = (uint16_t)plane[p];
             }
         }
-        if (tile * QP_TILE + row >= a.n) guard = 0;
+        if (tile * QP_TILE + row >= a.n || n2_s[row] == 0.0f) guard = 0;
         // ---- coordinates next to a boundary again, by the chain of quantize.cu: a warp per coordinate ----
         while (__syncthreads_or(guard != 0)) {
             while (guard) {
