@@ -96,8 +96,8 @@ def test_queries_that_tie_everywhere_stop_gathering():
     assert best_ms(zeros) < 4 * (lists + best_ms(q))         # (counting all of them took 48 times as long)
 
 
-def _in_shards(idx, q, k, rows=1000):
-    """The search of a Prod-mode index in shards of so few rows that the float32 list kernel ranks them."""
+def _in_shards(idx, q, k, rows=960):
+    """The search of a Prod-mode index in shards of so few rows that the float32 list kernel ranks them (whole tiles of 16)."""
     from turboquant_kv import TurboQuantIndex
     from turboquant_kv.search import merge_topk
 
@@ -126,7 +126,7 @@ def test_rows_and_queries_that_are_not_finite(mode, k):
         packed, norms = idx._packed_codes.clone(), idx._norms.clone()
     else:
         norms = idx._norms
-    norms[17::300] = float("inf")
+    norms[17::40] = float("inf")
     norms[30::500] = float("nan")
     if mode == "mse":
         idx._import_rows(packed, norms)
@@ -155,14 +155,14 @@ def test_prod_rows_that_half_precision_cannot_tell_apart(dim, k, nq):
     rows[::10] = rows[7]                                        # 3,000 copies
     idx = TurboQuantIndex(dim=dim, bit_width=3, mode="prod", seed=42)
     idx.add(rows)
-    idx._residual_norms[::10] *= 1 + 2e-3 * torch.rand(3000, generator=gen).cuda()
+    idx._residual_norms[::10] *= 1 + 1e-2 * torch.rand(3000, generator=gen).cuda()
     q = torch.cat([rows[7][None, :] + 0.3 * torch.randn((nq + 1) // 2, dim, generator=gen), torch.randn(nq // 2, dim, generator=gen)]).cuda()
     scores, ids = idx.search(q, k)
     want_s, want_i = _in_shards(idx, q, k)
     assert torch.equal(scores, want_s) and torch.equal(ids, want_i)
 
 
-@pytest.mark.parametrize("bits,k", [(4, 32), (2, 40), (4, 233), (3, 256)])
+@pytest.mark.parametrize("bits,k", [(4, 32), (2, 40), (3, 233), (3, 256)])
 def test_mse_rows_that_half_precision_cannot_tell_apart(bits, k):
     """Queries whose coordinates differ by less than fp16 resolves, rows that raise one of them each: for k > 24 the ranking keeps
     22 bits of the queries, whether a call has few or many."""
@@ -184,7 +184,7 @@ def test_mse_rows_that_half_precision_cannot_tell_apart(bits, k):
     assert torch.equal(scores, torch.cat([s for s, _ in few])) and torch.equal(ids, torch.cat([i for _, i in few]))
 
 
-@pytest.mark.parametrize("dim,bits,n,nq,k", [(128, 4, 40_003, 16, 233), (64, 3, 90_000, 40, 256), (128, 2, 70_001, 9, 240)])
+@pytest.mark.parametrize("dim,bits,n,nq,k", [(128, 3, 40_003, 16, 233), (64, 3, 90_000, 40, 256), (128, 2, 70_001, 9, 240)])
 def test_the_largest_k(dim, bits, n, nq, k):
     from turboquant_kv import TurboQuantIndex
 
