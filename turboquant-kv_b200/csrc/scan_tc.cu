@@ -16,7 +16,9 @@
 // passes.  Here a first launch scores every `stride`-th tile and keeps only the largest score of each group of rows; the
 // ksel-th largest of those maxima is not above the ksel-th best score of all rows (the maxima belong to distinct rows), and
 // the main launch appends every row that is not below it, about ksel * stride of them, to the query's buffer.  A query
-// whose buffer overflows (many rows tied with the bound) is scanned again by the list kernels, which other queries skip.
+// whose buffer overflows (many rows tied with the bound), or would by what the sample shows, is scanned by the list kernels,
+// which other queries skip; it gathers no further (32 queries, 28 of them zero, over 1 M rows: 17.5 ms with all tied rows
+// counted, 0.46 ms now, 0.37 ms by the list kernels alone).
 //
 // What bounds it (d = 128, 256 queries, clocks of a 128-row tile): 1,024 on the tensor cores, about 1,400 issue slots per
 // scheduler in the epilogue (a multiply-add, half a compare and a quarter of a shared load per score), 500 in the decoders.
@@ -113,9 +115,9 @@ __global__ void __launch_bounds__(128) scan_tc_image_kernel(const ScanTcArgs a) 
 __global__ void __launch_bounds__(256) scan_tc_threshold_kernel(const ScanTcArgs a) {
     extern __shared__ float g[];
     __shared__ float top[256], bound, low;
-    __shared__ int left;
+    __shared__ int left, reach;                            // reach: maxima not below the bound
     const int q = blockIdx.x, t = threadIdx.x;
-    if (t == 0) { bound = ST_NEG_INF; low = ST_NEG_INF; left = 0; }
+    if (t == 0) { bound = ST_NEG_INF; low = ST_NEG_INF; left = 0; reach = 0; }
     float v = ST_NEG_INF;
     for (int i = t; i < a.groups; i += 256) v = fmaxf(v, a.gmax[(int64_t)q * a.groups + i]);
     top[t] = v;
@@ -138,13 +140,30 @@ __global__ void __launch_bounds__(256) scan_tc_threshold_kernel(const ScanTcArgs
         if (r == a.rank - 1) bound = x;                    // (ranks are distinct)
     }
     __syncthreads();
+    for (int i = t; i < n; i += 256)
+        if (g[i] >= bound) atomicAdd(&reach, 1);
+    __syncthreads();
     if (t == 0) {
         // the main launch compares unrounded products with it: a little lower, so that the bound's own row stays (and finite,
         // so that infinite scores are not below it)
         a.thr[q] = fminf(bound, 3.4e38f) - fabsf(fminf(bound, 3.4e38f)) * 2e-6f;
-        // the list kernels answer where the sample gave up or gave no bound (rows or queries that are not numbers)
-        a.count[q] = a.limits[2] || bound == ST_NEG_INF ? a.cap + 1 : 0;
+        // The list kernels answer where the sample gave up, gave no bound (rows or queries that are not numbers), or tells that
+        // the buffer will overflow: each maximum that reaches the bound stands for a.stride rows at least, and without ties
+        // there are a.rank of them.
+        a.count[q] = a.limits[2] || bound == ST_NEG_INF || (int64_t)reach * a.stride > a.cap ? a.cap + 1 : 0;
     }
+}
+
+// ---- largest norm of the records (proven MSE calls; inside the main launch it cost the calls that need none 5 %) ----
+__global__ void __launch_bounds__(256) scan_tc_norms_kernel(const ScanTcArgs a) {
+    const int norms = a.rec_bytes - 64;                    // key-only records end with their sixteen norms
+    float top = 0.0f;
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < a.rows / 4; i += (int64_t)gridDim.x * 256) {
+        const float4 v = __ldg(reinterpret_cast<const float4*>(a.records + (i >> 2) * a.rec_bytes + norms) + (i & 3));
+        top = fmaxf(fmaxf(top, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));     // (NaN: passed over)
+    }
+    top = st_warp_max(top);
+    if ((threadIdx.x & 31) == 0) atomicMax(a.limits, __float_as_uint(top));
 }
 
 // ---- decoders ----------------------------------------------------------------------------------------
@@ -180,6 +199,8 @@ __global__ void __launch_bounds__(ST_THREADS, 1) scan_tc_kernel(const ScanTcArgs
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int q0 = blockIdx.y * a.cols;
     const int64_t ntiles = (a.rows + ST_TILE - 1) / ST_TILE;
+    // (a block of queries that all go to the list kernels has nothing to gather)
+    if (!SAMPLE && !__syncthreads_or(threadIdx.x < a.cols && q0 + (int)threadIdx.x < a.nq && a.count[q0 + threadIdx.x] <= a.cap)) return;
     const int64_t nwork = SAMPLE ? (ntiles + a.stride - 1) / a.stride : ntiles;
     auto tile_of = [&](int64_t u) { return SAMPLE ? u * a.stride : u; };
 
@@ -214,7 +235,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) scan_tc_kernel(const ScanTcArgs
     }
     float* const thr_s = reinterpret_cast<float*>(sm + C::OFF_THR);
     if (!SAMPLE)
-        for (int c = threadIdx.x; c < ST_MAX_COLS; c += ST_THREADS) thr_s[c] = c < a.cols && q0 + c < a.nq ? a.thr[q0 + c] : -ST_NEG_INF;
+        for (int c = threadIdx.x; c < ST_MAX_COLS; c += ST_THREADS) thr_s[c] = c < a.cols && q0 + c < a.nq && a.count[q0 + c] <= a.cap ? a.thr[q0 + c] : -ST_NEG_INF;
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -307,7 +328,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) scan_tc_kernel(const ScanTcArgs
             __syncwarp();
             if (lane == 0) st_arrive(a_ready(b));
         }
-        if (PROD && !SAMPLE && blockIdx.y == 0) {
+        if (PROD && !SAMPLE) {
             top_sign = st_warp_max(top_sign);
             if (lane == 0) atomicMax(a.limits + 1, __float_as_uint(top_sign));
         }
@@ -318,7 +339,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) scan_tc_kernel(const ScanTcArgs
         const uint32_t thr_at = base + C::OFF_THR + col0 * 4;
         uint32_t it = 0;
         float mine[4] = {ST_NEG_INF, ST_NEG_INF, ST_NEG_INF, ST_NEG_INF};       // SAMPLE: group maxima of columns 32 i + lane
-        float top_norm = 0.0f;                             // largest |norm| of the thread's rows
+        float top_norm = 0.0f;                             // Prod: largest |norm| of the thread's rows
         int flush = 0;
         auto put_group = [&]() {
 #pragma unroll
@@ -340,8 +361,8 @@ __global__ void __launch_bounds__(ST_THREADS, 1) scan_tc_kernel(const ScanTcArgs
                 if (at < a.cap) {
                     a.buf_s[(int64_t)q * a.cap + at] = __uint_as_float(log[3 * e + 1]);
                     a.buf_i[(int64_t)q * a.cap + at] = (int)log[3 * e + 2];
-                } else {                                   // overflowed: no more of this query's rows (32 queries, 28 of them zero,
-                    thr_s[q - q0] = -ST_NEG_INF;           // over 1 M rows: 17.5 ms where all were counted)
+                } else {
+                    thr_s[q - q0] = -ST_NEG_INF;           // overflowed: no more of this query's rows
                 }
             }
             __syncwarp();
@@ -354,7 +375,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) scan_tc_kernel(const ScanTcArgs
             if (r < a.rows)
                 nrm = PROD ? __ldg(a.norms + r)
                            : __ldg(reinterpret_cast<const float*>(a.records + (r >> 4) * a.rec_bytes + tl_key_section(D, BITS ? BITS : 4) + tl_norm_offset(0, 0, (int)(r & 15))));
-            if (!SAMPLE) top_norm = fmaxf(top_norm, fabsf(nrm));           // (NaN: passed over)
+            if (PROD && !SAMPLE) top_norm = fmaxf(top_norm, fabsf(nrm));   // (NaN: passed over)
             ok = mbar_wait(acc_full(b), (it >> 1) & 1);
             if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
             tc_fence_after();
@@ -427,7 +448,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) scan_tc_kernel(const ScanTcArgs
             while (flush < a.flushes) put_group();         // (what is left, then groups without rows)
         } else {
             take_places();
-            if (blockIdx.y == 0 && half == 0) {
+            if (PROD && half == 0) {                       // (every block sees every row)
                 top_norm = st_warp_max(top_norm);
                 if (lane == 0) atomicMax(a.limits, __float_as_uint(top_norm));
             }
@@ -530,6 +551,10 @@ static int st_launch(const ScanTcArgs& a, cudaStream_t st) {
     if (int e = check_launch("scan_tc_sample")) return e;
     scan_tc_threshold_kernel<<<a.nq, 256, a.groups * sizeof(float), st>>>(a);
     if (int e = check_launch("scan_tc_threshold")) return e;
+    if (!PROD && a.proven) {
+        scan_tc_norms_kernel<<<(unsigned)std::min<int64_t>(8 * sm_count(), ceil_div(a.rows, 1024)), 256, 0, st>>>(a);
+        if (int e = check_launch("scan_tc_norms")) return e;
+    }
     main_pass<<<grid_main, ST_THREADS, C::TOTAL, st>>>(a);
     return check_launch("scan_tc");
 }
