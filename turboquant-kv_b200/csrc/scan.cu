@@ -832,6 +832,8 @@ __global__ void __launch_bounds__(SCAN_WARPS * 32) scan_generic_kernel(const Sca
     int* lists_i = reinterpret_cast<int*>(lists_s + SCAN_WARPS * p.kk);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int q = blockIdx.y;
+    pdl_trigger();
+    pdl_wait();
     if (p.buf_n && p.buf_n[q] <= p.buf_cap) return;
     if (prod)
         for (int e = threadIdx.x; e < p.dim; e += blockDim.x) Ts[e] = p.qsign[(int64_t)q * p.dim + e];
@@ -1506,10 +1508,10 @@ extern "C" int tqb_scan_topk_prod(const float* queries, int nq, const uint8_t* m
     }
     const size_t smem = sizeof(float) * ((size_t)dim * (1 << mb) + dim) + (size_t)SCAN_WARPS * p.kk * 8;
     TQB_CUDA(cudaFuncSetAttribute(scan_generic_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    dim3 grid(gx, nq);
-    scan_generic_kernel<<<grid, SCAN_WARPS * 32, smem, st>>>(p);
+    // (after a proven selection these two have nothing to do for most queries: they are set up while their predecessors run)
+    TQB_CUDA(launch_pdl(p.proven, scan_generic_kernel, dim3(gx, nq), dim3(SCAN_WARPS * 32), smem, st, p));
     if (int e = check_launch("scan_generic")) return e;
-    return launch_merge(p, false, msmem, 0, st);
+    return launch_merge(p, false, msmem, p.proven, st);
 }
 
 extern "C" int tqb_topk_merge(const float* scores, const int64_t* ids, int nq, int parts, int k,
