@@ -192,3 +192,55 @@ def test_cache_update_keeps_the_tangent_of_new_tokens():
             assert ta is not None and tv is not None
             assert torch.equal(ta[:, :, old:], dk) and torch.equal(tv[:, :, old:], dv) and not ta[:, :, :old].any()
         assert torch.equal(ka[:, :, old:], k) and ka.shape[2] == old + T
+
+
+@pytest.mark.parametrize("prod", [False, True])
+@pytest.mark.parametrize("dim", [32, 64, 96, 128])
+def test_error_is_no_larger_than_the_ffma_kernels(dim, prod):
+    """Codes of normal rows: the relative error against 64-bit sums, of one large call and of calls that stay on the FFMA kernel."""
+    import turboquant_kv.reference as R
+
+    n = 20_000
+    gen = torch.Generator(device="cuda").manual_seed(dim)
+    rot, S = R.make_rotation_matrix(dim, 42).cuda(), R._make_qjl_matrix(dim, dim, 42, "cuda")
+    x = torch.randn(n, dim, generator=gen, device="cuda")
+    for bits in (2, 3, 4):
+        cb = tuple(t.cuda() for t in R.lloyd_max_codebook(bits - prod, dim))
+        if prod:
+            rows = R.quantize_prod(x, bits, rotation=rot, codebook=cb, S_matrix=S)
+            back = lambda lo, hi: R.dequantize_prod(*(t[lo:hi] for t in rows), bits, dim, rotation=rot, codebook=cb, S_matrix=S)
+        else:
+            rows = R.quantize_mse(x, bits, rotation=rot, codebook=cb)
+            back = lambda lo, hi: R.dequantize_mse(rows[0][lo:hi], rows[1][lo:hi], bits, dim, rotation=rot, codebook=cb)
+        want = cb[1].double()[R.unpack_codes(rows[0], bits - prod, dim).long()] @ rot.double()
+        if prod:
+            signs = R.unpack_codes(rows[1], 1, dim).double() * 2 - 1
+            want += math.sqrt(math.pi / 2) / dim * rows[2].double()[:, None] * (signs @ S.double())
+        want *= rows[-1].double()[:, None]
+        large = float((back(0, n).double() - want).norm() / want.norm())
+        small = float((torch.cat([back(lo, min(n, lo + 250)) for lo in range(0, n, 250)]).double() - want).norm() / want.norm())
+        assert large <= small, (bits, large, small)
+
+
+@pytest.mark.parametrize("dim,kb,vb", [(64, 4, 2), (64, 3, 3), (128, 4, 3), (128, 2, 4)])
+def test_error_of_records_is_no_larger_than_the_ffma_kernels(dim, kb, vb):
+    import turboquant_kv.reference as R
+    from turboquant_kv import _native as N
+    from turboquant_kv.kvstore import PackedKVStore
+
+    units, tokens = 8, 2000
+    gen = torch.Generator(device="cuda").manual_seed(dim + kb)
+    kv = PackedKVStore(dim, kb, vb, 42, "dense_qr", "cuda")
+    store = kv.alloc(units, tokens)
+    k, v = (torch.randn(units, tokens, dim, generator=gen, device="cuda") for _ in range(2))
+    k[..., :4] *= 20.0
+    rm = N.RowMap(tokens, tokens, 1, 0, None, 1, None, 1)
+    kv.append(store, k, v, rm)
+    kp, kn, vp, vn = kv.export_rows(store, units * tokens, rm)
+    got = kv.dequantize_units(store, units, tokens, tokens)
+    for g, which, p, nm, bits, cb, rot in ((got[0], "key", kp, kn, kb, kv.key_codebook, kv.key_rotation),
+                                           (got[1], "value", vp, vn, vb, kv.val_codebook, kv.val_rotation)):
+        want = (cb[1].double()[R.unpack_codes(p, bits, dim).long()] @ rot.double()) * nm.double()[:, None]
+        small = torch.cat([kv.dequantize(p[lo:lo + 250], nm[lo:lo + 250], which) for lo in range(0, units * tokens, 250)])
+        large, small = (float((t.double().view(-1, dim) - want).norm() / want.norm()) for t in (g, small))
+        assert large <= small, (which, large, small)

@@ -8,8 +8,10 @@
 // Arithmetic: float32.  Centroids, rotation and QJL matrix enter the MMAs as two fp16 terms each, hi = fp16(v) and
 // lo = fp16(v - hi), after scaling by a power of two that keeps the low terms out of the subnormal range: 22 bits
 // against float32's 24.  The three products that matter (lo hi, hi lo, then hi hi) are accumulated in float32; the
-// signs are exact in one term.  Measured against 64-bit sums: 2e-7 of a row's length, the float32 FMA chain's own
-// error.
+// signs are exact in one term.  The accumulator is rounded toward zero after every MMA, a loss in proportion to the
+// partial sum there, which the matrices' low terms give back (DQ_LOSS).  Relative error against 64-bit sums of
+// codes of normal rows, dims 32 to 128, 1 to 4 bits: 0.6 to 1.6e-7 (records with outlier channels among them), the float32
+// FMA chain of dequantize.cu 1.0 to 2.1e-7; without what DQ_LOSS gives back 0.9 to 2.9e-7.
 //
 // What bounds it: the shared-memory pipe.  A 128-row tile of d = 128 writes 64 KB of float32 (2,900 clocks of HBM at 22
 // bytes per clock and SM); it takes 24 MMAs that read 8 KB of operands each (1,536 clocks), 256 table loads and 64 KB of
@@ -33,6 +35,10 @@ namespace tqb {
 constexpr int DQ_TILE = 128;                 // rows per tile = TMEM lanes
 constexpr int DQ_DEC = 8, DQ_EPI = 8;        // decoder and epilogue warps
 constexpr int DQ_THREADS = (DQ_DEC + DQ_EPI + 1) * 32;
+// Mean loss of a truncation to 24 bits, relative to the number: half a unit of the last place, which is 2^-23 to 2^-24 of it
+// (0.36 2^-23 where all leading digits are as frequent as in products; measured 0.32).  A product added in step s of the
+// leading product's n is in n - s truncated sums, so its matrix element is scaled by 1 + DQ_LOSS (n - s).
+constexpr float DQ_LOSS = 0.32f * 1.1920929e-7f;
 
 struct DqSide {                              // one operand set: rows, or the keys or values of a record store
     const uint8_t* src;                      // packed rows, or the record store
@@ -107,16 +113,16 @@ __device__ __forceinline__ void transpose4(uint32_t (&v)[32], int lane) {
         }
     }
 }
-// v -> {hi, lo} fp16 terms
-__device__ __forceinline__ void split_half(float v, uint32_t& hi, uint32_t& lo) {
+// v (1 + more) -> {hi, lo} fp16 terms
+__device__ __forceinline__ void split_half(float v, uint32_t& hi, uint32_t& lo, float more = 0.0f) {
     const __half h = __float2half_rn(v);
-    const __half l = __float2half_rn(v - __half2float(h));
+    const __half l = __float2half_rn(fmaf(v, more, v - __half2float(h)));
     hi = __half_as_ushort(h); lo = __half_as_ushort(l);
 }
 // B operand of one matrix M (dim x dim, row j = contraction index): B[n][k = j] = M[j][n], K-major with 128-byte
-// swizzle, hi and lo terms.  All threads of the CTA; returns the scale.  red: 32 floats of scratch.
+// swizzle, hi and lo terms, scaled by 1 + gain.  All threads of the CTA; returns the scale.  red: 32 floats of scratch.
 template <int DP>
-__device__ __forceinline__ float build_b(uint8_t* sm, int off_hi, int off_lo, const float* __restrict__ M, int dim, float* red) {
+__device__ __forceinline__ float build_b(uint8_t* sm, int off_hi, int off_lo, const float* __restrict__ M, int dim, float gain, float* red) {
     constexpr int BLOCKS = (DP / 2) * (DP / 4);            // 2 rows x 4 columns each
     constexpr int PER = (BLOCKS + DQ_THREADS - 1) / DQ_THREADS;
     float4 r0[PER], r1[PER];
@@ -156,6 +162,7 @@ __device__ __forceinline__ float build_b(uint8_t* sm, int off_hi, int off_lo, co
         if (b >= BLOCKS) continue;
         int j, n;
         place(b, j, n);
+        const float more = fmaf(DQ_LOSS, (float)((dim + 15) / 16 - (j >> 4)), gain);      // (j and j + 1 are in one step of 16)
         const int turn = (b >> 3) & 3;                     // rotation of the four columns, by column group
 #pragma unroll
         for (int cc = 0; cc < 4; cc++) {
@@ -163,8 +170,8 @@ __device__ __forceinline__ float build_b(uint8_t* sm, int off_hi, int off_lo, co
             const float v0 = c & 2 ? (c & 1 ? r0[i].w : r0[i].z) : (c & 1 ? r0[i].y : r0[i].x);
             const float v1 = c & 2 ? (c & 1 ? r1[i].w : r1[i].z) : (c & 1 ? r1[i].y : r1[i].x);
             uint32_t h0, l0, h1, l1;
-            split_half(v0 * sc, h0, l0);
-            split_half(v1 * sc, h1, l1);
+            split_half(v0 * sc, h0, l0, more);
+            split_half(v1 * sc, h1, l1, more);
             const uint32_t off = (uint32_t)(j >> 6) * (DP * 128) + sw128_offset(n + c, j & 63);
             *reinterpret_cast<uint32_t*>(sm + off_hi + off) = h0 | (h1 << 16);
             *reinterpret_cast<uint32_t*>(sm + off_lo + off) = l0 | (l1 << 16);
@@ -290,16 +297,23 @@ __global__ void __launch_bounds__(DQ_THREADS, 1) dequantize_tc_kernel(const DqAr
     if (warp == DQ_DEC + DQ_EPI) tmem_alloc(smem_u32(&tmem_slot), C::TMEM_COLS);
 
     // ---- constants: the B operands, the pair table ----
-    float unscale = 1.0f / build_b<DP>(sm, C::OFF_B, C::OFF_B + C::B_TERM, sd.rot, a.dim, red), unscale_s = 1.0f;
-    if (PROD) unscale_s = 1.0f / build_b<DP>(sm, C::OFF_B + 2 * C::B_TERM, C::OFF_B + 3 * C::B_TERM, a.qjl, a.dim, red);
+    // What the terms of the centroids leave is the same for every coordinate of a code: the matrix takes it back on average.
+    float mx = 0.0f, left = 0.0f, square = 0.0f;
+    for (int i = 0; i < (1 << bits); i++) mx = fmaxf(mx, fabsf(__ldg(sd.cent + i)));
+    const float sc = fp16_scale(mx);
+    for (int i = 0; i < (1 << bits); i++) {
+        const float v = __ldg(sd.cent + i) * sc, h = __half2float(__float2half_rn(v)), l = __half2float(__float2half_rn(v - h));
+        left = fmaf(v - h - l, v, left);
+        square = fmaf(v, v, square);
+    }
+    const float gain = square > 0.0f && square < 1e30f ? left / square : 0.0f;
+    float unscale = 1.0f / build_b<DP>(sm, C::OFF_B, C::OFF_B + C::B_TERM, sd.rot, a.dim, gain, red), unscale_s = 1.0f;
+    if (PROD) unscale_s = 1.0f / build_b<DP>(sm, C::OFF_B + 2 * C::B_TERM, C::OFF_B + 3 * C::B_TERM, a.qjl, a.dim, 0.0f, red);
+    unscale *= 1.0f / sc;
     const int entries = 1 << (2 * bits);
     int shift = 3;                                             // entry stride = 8 bytes x copies (up to 8)
     while (shift < 6 && (entries << (shift + 1)) <= C::LUT) shift++;
     {
-        float mx = 0.0f;
-        for (int i = 0; i < (1 << bits); i++) mx = fmaxf(mx, fabsf(__ldg(sd.cent + i)));
-        const float sc = fp16_scale(mx);
-        unscale *= 1.0f / sc;
         for (int e = threadIdx.x; e < (entries << (shift - 3)); e += DQ_THREADS) {
             const int x = e >> (shift - 3);
             int c0, c1;                                        // codes of the pair's first and second element
