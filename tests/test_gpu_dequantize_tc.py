@@ -244,3 +244,32 @@ def test_error_of_records_is_no_larger_than_the_ffma_kernels(dim, kb, vb):
         small = torch.cat([kv.dequantize(p[lo:lo + 250], nm[lo:lo + 250], which) for lo in range(0, units * tokens, 250)])
         large, small = (float((t.double().view(-1, dim) - want).norm() / want.norm()) for t in (g, small))
         assert large <= small, (which, large, small)
+
+
+@pytest.mark.parametrize("prod", [False, True])
+@pytest.mark.parametrize("dim", [64, 96, 128])
+@pytest.mark.parametrize("norm", [1e-35, 1e30])
+def test_extreme_norms_keep_their_digits(dim, norm, prod):
+    """The norm multiplies the sum, not the operands' scale, which would leave it few bits below float32's normal range."""
+    import turboquant_kv.reference as R
+
+    n = 600
+    gen = torch.Generator(device="cuda").manual_seed(dim)
+    rot, S = R.make_rotation_matrix(dim, 42).cuda(), R._make_qjl_matrix(dim, dim, 42, "cuda")
+    cent = R.lloyd_max_codebook(3, dim)[1].cuda()
+    codes = torch.randint(0, 8, (n, dim), generator=gen, device="cuda", dtype=torch.uint8)
+    norms = torch.rand(n, generator=gen, device="cuda") + 0.5
+    norms[100:300] *= norm
+    norms[400] = 0.0
+    want = cent.double()[codes.long()] @ rot.double()
+    length = want.norm(dim=1)
+    if prod:
+        sg, rn = torch.randint(0, 2, (n, dim), generator=gen, device="cuda", dtype=torch.uint8), torch.rand(n, generator=gen, device="cuda")
+        coef = math.sqrt(math.pi / 2) / dim * rn.double()
+        want += coef[:, None] * ((sg.double() * 2 - 1) @ S.double())
+        length += coef * S.double().abs().sum(0).max()
+        got = R.dequantize_prod(R.pack_codes(codes, 3), R.pack_codes(sg, 1), rn, norms, 4, dim, rotation=rot, codebook=(None, cent), S_matrix=S)
+    else:
+        got = R.dequantize_mse(R.pack_codes(codes, 3), norms, 3, dim, rotation=rot, codebook=(None, cent))
+    err = (got.double() - want * norms.double()[:, None]).abs()
+    assert bool((err <= (EPS * length * norms.double())[:, None] + 2.0 ** -149).all()) and not got[400].any()

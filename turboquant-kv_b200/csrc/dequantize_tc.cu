@@ -438,6 +438,8 @@ __global__ void __launch_bounds__(DQ_THREADS, 1) dequantize_tc_kernel(const DqAr
         const int ew = warp & 3, half = (warp - DQ_DEC) >> 2;
         const int row = ew * 32 + lane, col0 = half * (DP / 2);
         // 32 accumulator columns -> scaled float32
+        float nrm = 0.0f;
+        bool small = false;                                    // a row of the warp has so small a norm that f would lose digits
         auto load_cols = [&](uint32_t taddr, float f, float fs, uint32_t (&v)[32]) {
             tmem_ld32(taddr, v);
             if (PROD) {
@@ -448,6 +450,10 @@ __global__ void __launch_bounds__(DQ_THREADS, 1) dequantize_tc_kernel(const DqAr
             } else {
 #pragma unroll
                 for (int i = 0; i < 32; i++) v[i] = __float_as_uint(__uint_as_float(v[i]) * f);
+            }
+            if (small) {
+#pragma unroll
+                for (int i = 0; i < 32; i++) v[i] = __float_as_uint(__uint_as_float(v[i]) * nrm);
             }
         };
         auto pack_cols = [&](uint32_t (&v)[32]) {
@@ -461,8 +467,9 @@ __global__ void __launch_bounds__(DQ_THREADS, 1) dequantize_tc_kernel(const DqAr
         uint32_t it = 0;
         for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, it++) {
             const int b = it & 1;
-            float nrm = 0.0f, coef = 0.0f;
+            float coef = 0.0f;
             int64_t orow = -1;
+            nrm = 0.0f;
             if (RECORDS) {
                 const int64_t rec = tile * 8 + (row >> 4);
                 if (rec < a.n) {
@@ -489,7 +496,8 @@ __global__ void __launch_bounds__(DQ_THREADS, 1) dequantize_tc_kernel(const DqAr
             int64_t rows4[4];
 #pragma unroll
             for (int i = 0; i < 4; i++) rows4[i] = __shfl_sync(0xffffffffu, orow, (lane & ~3) + i);
-            const float f = unscale * nrm, fs = coef * nrm;
+            small = __any_sync(0xffffffffu, nrm != 0.0f && fabsf(unscale * nrm) < 1e-30f);
+            const float f = small ? unscale : unscale * nrm, fs = small ? coef : coef * nrm;
             // 32 columns of float32, or 64 of a 16-bit type: 128 bytes of every row a turn
             const bool half_out = a.out_dtype != TQB_F32;
             const int turn = half_out && DP / 2 >= 64 ? 64 : 32;
