@@ -12,7 +12,16 @@ from util import MAX_TIE_RATE, code_mismatches
 
 pytestmark = pytest.mark.gpu
 
-SMALL = 256     # rows per call that stay on the FFMA kernel (the tensor-core path starts at 512)
+SMALL = 256     # rows per call that stay on the FFMA kernel
+
+
+def _large() -> int:
+    """Rows of a single-tensor call that is well above the FFMA kernel's short-call rule (one row a warp up to 32 rows an SM), in
+    128-row tiles of which the last is ragged."""
+    rule = 32 * torch.cuda.get_device_properties(0).multi_processor_count
+    n = rule + 4 * 128 + 3
+    assert n > rule and n % 128
+    return n
 
 
 def _rows(n, dim, dtype, seed, outliers=True):
@@ -36,7 +45,7 @@ def _status():
 def test_tensor_core_quantise_equals_ffma_kernel_and_oracle(orc, dtype, dim, bits):
     import turboquant_kv.reference as R
 
-    n = 4 * 1024 + 3                    # 33 tiles, the last one ragged
+    n = _large()
     x = _rows(n, dim, dtype, seed=dim + bits)
     rot = orc.make_rotation_matrix(dim, 42)
     bnd, cent = orc.lloyd_max_codebook(bits, dim)
@@ -82,7 +91,8 @@ def test_tensor_core_append_writes_the_same_records(dim, kb, vb):
     from turboquant_kv import _native as N
     from turboquant_kv.kvstore import PackedKVStore
 
-    units, tokens = 6, 700              # rows are (unit, token): 4,200 rows per call
+    units, tokens = 6, 700              # rows are (unit, token): 4,200 rows of two tensors per call
+    assert 2 * units * tokens > 32 * torch.cuda.get_device_properties(0).multi_processor_count
     kv = PackedKVStore(dim, kb, vb, 42, "dense_qr", "cuda")
     k = _rows(units * tokens, dim, torch.bfloat16, seed=1).view(units, tokens, dim)
     v = _rows(units * tokens, dim, torch.bfloat16, seed=2, outliers=False).view(units, tokens, dim)
@@ -140,7 +150,7 @@ def test_tensor_core_quantise_strided_rows(orc):
     """Rows that are not contiguous (x_stride > dim) go through one TMA copy per row."""
     from turboquant_kv import _native as N
 
-    n, dim, bits, stride = 2048, 128, 4, 160
+    n, dim, bits, stride = _large(), 128, 4, 160
     buf = torch.randn(n, stride, generator=torch.Generator().manual_seed(3)).cuda()
     rot = torch.from_numpy(orc.make_rotation_matrix(dim, 42)).cuda()
     bnd, _ = orc.lloyd_max_codebook(bits, dim)
@@ -157,3 +167,8 @@ def test_tensor_core_quantise_strided_rows(orc):
     torch.cuda.synchronize()
     assert _status() == 0
     assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+    import turboquant_kv.reference as R
+
+    how = {"rotation": rot, "codebook": (bnd_d, None)}
+    parts = [R.quantize_mse(buf[lo:lo + SMALL, :dim].contiguous(), bits, **how) for lo in range(0, n, SMALL)]
+    assert torch.equal(outs[0][0], torch.cat([p for p, _ in parts])) and torch.equal(outs[0][1], torch.cat([m for _, m in parts]))
