@@ -632,9 +632,9 @@ def extras(torch, dist, args, rank: int, world: int, device) -> dict:
             "prod_3bit_d128_vectors_per_s": 1_000_000 / (ms_p * 1e-3),
             "prod_3bit_estimator_bias": float((est - exact).mean()), "prod_3bit_estimator_slope": slope,
             "prod_3bit_search_1m_rows_64_queries_qps": 64 / (ms_ps * 1e-3), "prod_3bit_search_top10_overlap_with_exact_search": recall,
-            "note": "rank 0 only; MSE calls of 512 rows and more run the rotation on tcgen05 (bf16 operand splits, "
-                    "float32 accumulation in tensor memory, rows fed by TMA bulk copies), with the codes of the float32 "
-                    "FMA kernel; Prod mode and short calls run the float32 FMA kernel"}
+            "note": "rank 0 only; MSE calls of more than 32 rows an SM run the rotation on tcgen05 (bf16 operand splits, "
+                    "float32 accumulation in tensor memory, rows fed by TMA bulk copies), Prod calls of more than 8 rows an SM "
+                    "both projections (fp16 splits), with the codes of the float32 FMA kernel, which short calls run"}
         del db, x, est, exact
         torch.cuda.empty_cache()
 
@@ -690,8 +690,10 @@ def extras(torch, dist, args, rank: int, world: int, device) -> dict:
     sc_h, ids_h = index.search(hq, k)
     torch.cuda.synchronize()
     ms_host = sync_max((time.perf_counter() - t0) * 1e3)
-    per_pass = 8 if nq > 4 else 4        # calls with more than four queries take eight per pass (one fp16 column each)
-    passes = math.ceil(nq / per_pass)
+    # queries that share a read of the records: 4 (or 8) in the list kernel, from nine on a block of up to 256 on the tensor cores,
+    # in calls of at most 1,024 (the blocks of a call run side by side)
+    per_pass = 256 if nq >= 9 else 8 if nq > 4 else 4
+    passes = sum(math.ceil(min(1024, nq - c) / per_pass) for c in range(0, nq, 1024))
     scan_parity = None
     if world == 1 and not args.no_cpu and args.scan_parity_queries > 0:
         scan_parity = scan_reference_check(torch, index.local, queries[:args.scan_parity_queries], sc, ids, k)
