@@ -203,7 +203,7 @@ __device__ __forceinline__ uint32_t sign_pair(uint32_t w, int m, int u) {
 // Records: one warp per record.  `E` table entries: fields are little-endian code | code << bits pairs.
 template <int D, int BITS>
 struct RecChunk {
-    static constexpr int L = D * BITS / 16, NW = L / 4;    // bytes of a lane's chunk, words
+    static constexpr int L = D * BITS / 16;                // bytes of a lane's chunk
 };
 template <int D, int BITS>
 __device__ __forceinline__ void load_rec_key(const uint8_t* rec, int lane, uint32_t (&w)[D / 16]) {

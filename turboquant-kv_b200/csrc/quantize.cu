@@ -252,8 +252,9 @@ static int launch_quantize(const QuantArgs& a0, const QuantArgs& a1, int ntensor
 }
 
 // One row a warp, up to four waves of blocks.  Key-value append of n rows, device time: n = 32 d = 64 15 -> 5 us, d = 128
-// 34 -> 10 us; n = 592 (tensor-core kernel from 512 rows) 32 -> 5, 52 -> 10; n = 2,368 33 -> 11, 58 -> 27 (float32 38 -> 27).
-// One wave where a block holds (Prod: two matrices, one block an SM) or streams (dim > 128) more of them.
+// 34 -> 10 us; n = 592 (tensor-core kernel from 512 rows before) 32 -> 5, 52 -> 10; n = 2,368 33 -> 11, 58 -> 27 (float32 38 -> 27).
+// The line is where that sweep ended, not where the two cross: at 2,400 rows the tensor-core kernel takes 36 and 58 us, and a
+// wave of 592 rows more costs this one 2.5 (d = 64) to 5.5 us.  One wave where a block holds (Prod: two matrices, one block an SM) or streams (dim > 128) more of them.
 static bool few_rows(int64_t n, int tensors, int dim, bool prod) { return n * tensors <= (int64_t)sm_count() * (prod || dim > 128 ? 8 : 32); }
 
 template <typename T, bool PROD, int RW>

@@ -530,8 +530,10 @@ static int st_stride(int64_t rows, int ksel) { return (int)std::max<int64_t>(1, 
 
 bool scan_tc_wanted(int nq, int64_t rows, int dim, int bits, bool prod, int ksel, bool proven) {
     if ((dim != 64 && dim != 128) || bits < (prod ? 1 : 2) || bits > 4) return false;
-    // Two groups of rows per wanted candidate at least.  From nine queries (two passes of the list kernels) on: 8 queries over
-    // 1 M x d128 rows 207 us there, 16 here 124 us; 5,000 rows, 30 queries 141 us there.  Prod rows: the list kernel scores a row a lane.
+    // Two groups of rows per wanted candidate at least.  From nine queries (two passes of the list kernels) on: 9 queries over
+    // 2,300, 5,000 and 20,000 x d128 rows 127, 111 and 133 us there, 65 here.  Five to eight (one pass) are left to the list
+    // kernels although 8 queries over 1 M rows take 207 us there and 16 take 124 here.  Prod rows: the list kernel scores a row a
+    // lane; one query over 2,176 rows 74 us there, 66 here, over 30,000 360 and 67.
     if (4 * (rows / ST_TILE) < 2 * ksel) return false;
     // (a proof wants room below the k-th best score: twice the groups where k is large against the margin)
     if (proven && ksel > 64 && 4 * (rows / ST_TILE) < 4 * ksel) return false;
