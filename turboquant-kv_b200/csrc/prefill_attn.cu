@@ -796,6 +796,10 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const PrefillPar
             }
             if (ok) put_rotation(1);
         }
+        // a bulk copy still in flight must not outlive the block: the waits are bounded here too
+        if (!ok && dw == 0 && lane == 0)
+            for (uint32_t i = seq > PF_RING ? seq - PF_RING : 0; i < seq; i++) (void)mbar_wait(full(i % PF_RING), (i / PF_RING) & 1);
+        __syncwarp();
     } else if (lane == 0) {
         // ================= MMA issuer (one lane) =================
         constexpr uint32_t IDESC_M = (1u << 4) | ((uint32_t)(PF_ROWS >> 4) << 24);     // fp16 x fp16 -> f32, 128 rows
