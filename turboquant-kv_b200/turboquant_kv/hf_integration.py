@@ -21,7 +21,7 @@ import weakref
 from typing import Any, Dict, List, Optional, Tuple
 
 import torch
-from torch.autograd.forward_ad import unpack_dual
+from torch.autograd import forward_ad
 
 from . import _native as N
 from .config import TurboQuantConfig
@@ -38,9 +38,12 @@ except ImportError:  # pragma: no cover
     pass
 
 
-def _differentiated(*states: torch.Tensor) -> bool:
+def _differentiated(key: torch.Tensor, value: torch.Tensor) -> bool:
     """Whether a gradient (reverse mode) or a tangent (forward mode) flows through the states."""
-    return any((t.requires_grad and torch.is_grad_enabled()) or unpack_dual(t).tangent is not None for t in states)
+    if (key.requires_grad or value.requires_grad) and torch.is_grad_enabled():
+        return True
+    # (a tangent exists inside a dual level only; unpacking costs 2 us a tensor)
+    return getattr(forward_ad, "_current_level", 0) >= 0 and any(forward_ad.unpack_dual(t).tangent is not None for t in (key, value))
 
 
 class _LayerQuantStore:
@@ -68,15 +71,17 @@ class _LayerQuantStore:
             new[:, : self._store.shape[1]] = self._store
         self._store, self.capacity = new, cap
 
-    def _check(self, key: torch.Tensor, value: torch.Tensor) -> None:
-        B, H, D = self.batch, self.num_heads, self.head_dim
-        if key.dim() != 4 or value.shape != key.shape or key.shape[:2] != (B, H) or key.shape[3] != D:
-            raise RuntimeError(f"the layer holds ({B}, {H}, tokens, {D}) states, got keys {tuple(key.shape)} and values {tuple(value.shape)}")
+    def _new_tokens(self, key: torch.Tensor, value: torch.Tensor) -> int:
+        shape = key.shape
+        if (len(shape) != 4 or value.shape != shape or shape[0] != self.batch or shape[1] != self.num_heads
+                or shape[3] != self.head_dim):
+            raise RuntimeError(f"the layer holds ({self.batch}, {self.num_heads}, tokens, {self.head_dim}) states, got keys "
+                               f"{tuple(shape)} and values {tuple(value.shape)}")
+        return shape[2]
 
     def append(self, key: torch.Tensor, value: torch.Tensor) -> None:
         """key / value: (batch, heads, new, head_dim)."""
-        self._check(key, value)
-        T = key.shape[2]
+        T = self._new_tokens(key, value)
         self._reserve(self.seq_len + T)
         rm = N.RowMap(T, self.capacity, 1, self.seq_len, None, 1, None, 1)
         self.kv.append(self._store, key, value, rm)
@@ -85,8 +90,7 @@ class _LayerQuantStore:
     def update(self, key: torch.Tensor, value: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
         """``append``, and the dense history: (batch, heads, total, head_dim) keys and values in the inputs' dtype, old tokens
         dequantised, new tokens exact."""
-        self._check(key, value)
-        dt, T = key.dtype, key.shape[2]
+        dt, T = key.dtype, self._new_tokens(key, value)
         if (dt in (torch.float32, torch.float16, torch.bfloat16) and value.dtype == dt and key.device == self.device
                 and value.device == self.device and key.stride(3) == 1 and value.stride(3) == 1):
             self._reserve(self.seq_len + T)
