@@ -12,8 +12,9 @@
 // What bounds it (d = 128, float32, 2 bits + sign; clocks of a 128-row tile on one SM): 2 x 1,536 on the tensor cores, 2,600
 // issue slots for the exact divisions, 3,200 for code selection and residual terms, 1,300 of HBM: the phases of a tile
 // depend on one another and shared memory (both matrices, 128 KB, and one tile's terms) holds no second tile, so the
-// sixteen warps go through them together and only the loads run ahead.  Measured: 1 M rows 4.1 ms on the FFMA kernel, 0.65 ms
-// here (53 tiles an SM, 12 us each).
+// sixteen warps go through them together and only the loads run ahead.  Measured: 1 M rows 4.1 ms on the FFMA kernel, 0.71 ms
+// here (53 tiles an SM, 13 us each, 1 of them for the coordinates computed again: issuing the projection before those instead
+// of behind them cost more than it hid, 0.82 ms).
 #include "common.cuh"
 #include "pipe.cuh"
 #include "tc.cuh"
